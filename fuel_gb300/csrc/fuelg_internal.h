@@ -177,6 +177,25 @@ struct ExactScanParams {
 // out_keys [m, kk] (device).  Unused slots hold ~0ull.
 int exact_topk(const ExactScanParams& p, uint64_t* out_keys, int* dev_status, cudaStream_t stream);
 
+// The register-tiled form of the scan (fuelg_scan.cu) for KIND_KNN with the
+// shapes it takes; same keys as exact_topk, n >= 1.
+bool tile_scan_supported(int d, int kk);
+int tile_scan_topk(const ExactScanParams& p, uint64_t* out_keys, int* dev_status, cudaStream_t stream);
+// T tiles cut into G contiguous equal runs: run c's first tile, and the run that
+// holds tile t.
+#ifdef __CUDACC__
+#define FUELG_HD __host__ __device__
+#else
+#define FUELG_HD
+#endif
+FUELG_HD inline int64_t scan_run_begin(int64_t c, int64_t T, int64_t G) { return c * T / G; }
+FUELG_HD inline int64_t scan_run_of(int64_t t, int64_t T, int64_t G) { return ((t + 1) * G - 1) / T; }
+// Sorts the rows of unsorted kept keys that the tile scan's runs wrote (lists
+// [qblocks][J][qm][kk], kk <= 256, J <= 128) and merges each query's into keys
+// [m][kk]; lists == keys: one run per block, sorted in place.
+int sort_and_merge_runs(uint64_t* lists, int64_t m, int qm, int64_t nt, int64_t T, int64_t G, int J, int kk,
+                        uint64_t* keys, cudaStream_t stream);
+
 // Turn sorted keys [m, kk] into the reference's (int64 idx, float dist) rows
 // with the given exclude-self mode and -1/+inf padding.
 int finalize_knn(const uint64_t* keys, int64_t m, int kk, int k, int exclude_mode, int64_t* out_idx, float* out_dist,

@@ -26,6 +26,7 @@
 
 #include "fuelg_common.cuh"
 #include "fuelg_internal.h"
+#include "fuelg_select.cuh"
 #include "fuelg_tc_common.cuh"
 
 namespace fuelg {
@@ -71,7 +72,6 @@ struct KnnTcArgs {
 };
 
 
-constexpr int kSel = 8;  // keys per lane in a selection (appended or prefix): 256 per warp
 constexpr float kF16Max = 65504.0f;  // largest finite FP16 value
 
 // Screened keys kept for a query of k neighbours: k plus the margin the
@@ -81,104 +81,6 @@ constexpr float kF16Max = 65504.0f;  // largest finite FP16 value
 __host__ __device__ __forceinline__ int kk2_of(int k, int mode) {
   const int m = mode == 0 ? 0 : (mode == 1 ? k / 8 : k / 4);
   return mode == 0 ? k : k + (m > 8 ? m : 8);
-}
-
-// Number of held keys below t over the warp.
-__device__ __forceinline__ int warp_count_hi_below(const uint32_t (&hi)[2 * kSel], uint32_t t) {
-  int c = 0;
-#pragma unroll
-  for (int i = 0; i < 2 * kSel; i++) c += hi[i] < t ? 1 : 0;
-  return __reduce_add_sync(0xffffffffu, c);
-}
-
-// Warp-cooperative selection for one query: the union of its
-// na (<= 256) appended keys and its plen (<= kk <= 256) kept keys is reduced
-// to its kk smallest, written unsorted back over cur[0, min(kk, na + plen)).
-// The kk-th smallest key is found by a bitwise binary search over the
-// distance word (counting with a warp reduction) and, only when several keys
-// share that distance, over the index word; keys are unique.  Each search
-// starts below the bits that the smallest and largest candidate word share.
-// In place: every lane has read its keys before the first warp-wide
-// exchange, and every store comes after the last.  No shared memory, no sort.
-// Returns the kk-th smallest key, or KEY_NONE while fewer than kk are held,
-// on every lane.
-__device__ __noinline__ uint64_t warp_select(const uint64_t* __restrict__ app, int na, uint64_t* cur, int plen,
-                                             int kk, int lane) {
-  uint64_t key[2 * kSel];
-#pragma unroll
-  for (int i = 0; i < kSel; i++) {
-    const int e = lane + 32 * i;
-    key[i] = e < na ? app[e] : KEY_NONE;
-    key[kSel + i] = e < plen ? cur[e] : KEY_NONE;
-  }
-  uint32_t hi[2 * kSel];
-  uint32_t hmin = 0xffffffffu, hmax = 0;
-#pragma unroll
-  for (int i = 0; i < 2 * kSel; i++) {
-    hi[i] = (uint32_t)(key[i] >> 32);
-    if (key[i] != KEY_NONE) {
-      hmin = min(hmin, hi[i]);
-      hmax = max(hmax, hi[i]);
-    }
-  }
-  const int total = na + plen;
-  uint64_t kth = KEY_NONE;
-  if (total >= kk) {
-    // the kk-th distance word lies in [hmin, hmax]: search the bits below
-    // their common prefix only
-    hmin = __reduce_min_sync(0xffffffffu, hmin);
-    hmax = __reduce_max_sync(0xffffffffu, hmax);
-    int top = hmin == hmax ? -1 : 31 - __clz(hmin ^ hmax);
-    uint32_t H = top >= 0 ? hmin & ~((2u << top) - 1u) : hmin;
-    for (int b = top; b >= 0; b--) {
-      const uint32_t t = H | (1u << b);
-      if (warp_count_hi_below(hi, t) < kk) H = t;
-    }
-    // keys below H: fewer than kk; keys with hi == H: the rest is taken from them
-    const int below = warp_count_hi_below(hi, H);
-    int eq = 0;
-    uint32_t lmin = 0xffffffffu, lmax = 0;
-#pragma unroll
-    for (int i = 0; i < 2 * kSel; i++)
-      if (hi[i] == H) {
-        eq++;
-        lmin = min(lmin, (uint32_t)key[i]);
-        lmax = max(lmax, (uint32_t)key[i]);
-      }
-    eq = __reduce_add_sync(0xffffffffu, eq);
-    lmax = __reduce_max_sync(0xffffffffu, lmax);
-    const int need = kk - below;
-    uint32_t Lo = lmax;
-    if (eq != need) {
-      lmin = __reduce_min_sync(0xffffffffu, lmin);
-      top = lmin == lmax ? -1 : 31 - __clz(lmin ^ lmax);
-      Lo = top >= 0 ? lmin & ~((2u << top) - 1u) : lmin;
-      for (int b = top; b >= 0; b--) {
-        const uint32_t t = Lo | (1u << b);
-        int c = 0;
-#pragma unroll
-        for (int i = 0; i < 2 * kSel; i++) c += (hi[i] == H && (uint32_t)key[i] < t) ? 1 : 0;
-        if (__reduce_add_sync(0xffffffffu, c) < need) Lo = t;
-      }
-    }
-    kth = ((uint64_t)H << 32) | Lo;
-  }
-  // compact the kept keys: lane offsets by a warp scan of per-lane counts
-  int mine = 0;
-#pragma unroll
-  for (int i = 0; i < 2 * kSel; i++) mine += (key[i] != KEY_NONE && key[i] <= kth) ? 1 : 0;
-  int incl = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  int pos = incl - mine;
-#pragma unroll
-  for (int i = 0; i < 2 * kSel; i++)
-    if (key[i] != KEY_NONE && key[i] <= kth) cur[pos++] = key[i];
-  __syncwarp();
-  return total >= kk ? kth : KEY_NONE;
 }
 
 // 16-way register select without local memory: v[j] for a runtime j.
@@ -243,25 +145,17 @@ __global__ void __launch_bounds__(256) sort_rows_kernel(uint64_t* __restrict__ k
 
 constexpr int kMaxSplits = 128;
 
-// One warp per query: k-way merge of the sorted lists its query block's
-// pieces kept -- piece p holds rows in[p][0, QM)[0, kk2); the block's pieces are
-// [qb_pb[qb], qb_pb[qb + 1]), at most kMaxSplits -- into out[q][0, kk2); lane l
-// owns pieces l, l+32, ...
-__global__ void __launch_bounds__(256) merge_tc_splits_kernel(const uint64_t* __restrict__ in, int64_t m,
-                                                              const int32_t* __restrict__ qb_pb, int kk2,
-                                                              uint64_t* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (q >= m) return;
-  const int64_t qb = q / QM, row = q - qb * QM;
-  const int p0 = qb_pb[qb], S = qb_pb[qb + 1] - p0;
+// k-way merge by one warp of S <= kMaxSplits sorted lists of kk2 keys, list s at
+// in + s * stride, into out[0, kk2); lane l owns lists l, l+32, ...
+__device__ __forceinline__ void merge_sorted_lists(const uint64_t* __restrict__ in, size_t stride, int S, int kk2,
+                                                   uint64_t* __restrict__ out, int lane) {
   int pos[kMaxSplits / 32];
   uint64_t head[kMaxSplits / 32];
 #pragma unroll
   for (int t = 0; t < kMaxSplits / 32; t++) {
     const int sp = lane + 32 * t;
     pos[t] = 0;
-    head[t] = sp < S ? in[((size_t)(p0 + sp) * QM + row) * kk2] : KEY_NONE;
+    head[t] = sp < S ? in[(size_t)sp * stride] : KEY_NONE;
   }
   for (int j = 0; j < kk2; j++) {
     uint64_t mn = head[0];
@@ -273,16 +167,42 @@ __global__ void __launch_bounds__(256) merge_tc_splits_kernel(const uint64_t* __
                          __shfl_xor_sync(0xffffffffu, (uint32_t)mn, o);
       mn = v < mn ? v : mn;
     }
-    if (lane == 0) out[(size_t)q * kk2 + j] = mn;
+    if (lane == 0) out[j] = mn;
     if (mn == KEY_NONE) continue;
 #pragma unroll
     for (int t = 0; t < kMaxSplits / 32; t++)
       if (head[t] == mn) {  // keys are unique: one list advances
         const int sp = lane + 32 * t;
         pos[t]++;
-        head[t] = pos[t] < kk2 ? in[((size_t)(p0 + sp) * QM + row) * kk2 + pos[t]] : KEY_NONE;
+        head[t] = pos[t] < kk2 ? in[(size_t)sp * stride + pos[t]] : KEY_NONE;
       }
   }
+}
+
+// One warp per query: the sorted lists its query block's pieces kept -- piece
+// p holds rows in[p][0, QM)[0, kk2); the block's pieces are [qb_pb[qb],
+// qb_pb[qb + 1]), at most kMaxSplits -- merged into out[q][0, kk2).
+__global__ void __launch_bounds__(256) merge_tc_splits_kernel(const uint64_t* __restrict__ in, int64_t m,
+                                                              const int32_t* __restrict__ qb_pb, int kk2,
+                                                              uint64_t* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (q >= m) return;
+  const int64_t qb = q / QM, row = q - qb * QM;
+  const int p0 = qb_pb[qb], S = qb_pb[qb + 1] - p0;
+  merge_sorted_lists(in + ((size_t)p0 * QM + row) * kk2, (size_t)QM * kk2, S, kk2, out + (size_t)q * kk2, lane);
+}
+
+// The same for the runs of the FP32 tile scan (sort_and_merge_runs).
+__global__ void __launch_bounds__(256) merge_runs_kernel(const uint64_t* __restrict__ in, int64_t m, int qm,
+                                                         int64_t nt, int64_t T, int64_t G, int J, int kk,
+                                                         uint64_t* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (q >= m) return;
+  const int64_t qb = q / qm, row = q - qb * qm;
+  const int S = (int)(scan_run_of((qb + 1) * nt - 1, T, G) - scan_run_of(qb * nt, T, G)) + 1;
+  merge_sorted_lists(in + ((size_t)qb * J * qm + row) * kk, (size_t)qm * kk, S, kk, out + (size_t)q * kk, lane);
 }
 
 __global__ void __launch_bounds__(kThreadsKT, kCtasPerSm)
@@ -770,6 +690,19 @@ __global__ void scatter_keys_kernel(const uint64_t* __restrict__ src, int kk, in
 }
 
 }  // namespace
+
+int sort_and_merge_runs(uint64_t* lists, int64_t m, int qm, int64_t nt, int64_t T, int64_t G, int J, int kk,
+                        uint64_t* keys, cudaStream_t stream) {
+  const int64_t rows = lists == keys ? m : (m + qm - 1) / qm * J * qm;
+  sort_rows_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, stream>>>(lists, rows, kk);
+  note_launch();
+  if (lists != keys) {
+    merge_runs_kernel<<<(unsigned)((m * 32 + 255) / 256), 256, 0, stream>>>(lists, m, qm, nt, T, G, J, kk, keys);
+    note_launch();
+  }
+  FUELG_CUDA(cudaGetLastError());
+  return ST_OK;
+}
 
 namespace {
 // Shared memory of knn_tc_kernel without the B stages.
