@@ -166,6 +166,8 @@ struct fuelg_index {
   TcIndex* tc = nullptr;  // tensor-core form, built on the first tensor-core call
   bool f64 = false;       // a float64 index (fuelg_index_create_f64): X64 instead of X
   double* X64 = nullptr;  // device copy [n, d]
+  F64Screen* screen = nullptr;  // its rounded copy, built by the first kNN call
+  bool screen_tried = false;
   cudaStream_t stream = nullptr;
   std::mutex mu;  // calls on one handle are serialised
 };
@@ -494,6 +496,7 @@ int fuelg_index_destroy(fuelg_index* ix) {
   knn_tc_index_free(ix->tc);
   if (ix->X) cudaFree(ix->X);
   if (ix->X64) cudaFree(ix->X64);
+  f64_screen_free(ix->screen);
   if (ix->stream) cudaStreamDestroy(ix->stream);
   delete ix;
   return ST_OK;
@@ -1096,6 +1099,7 @@ int check_f64_index(fuelg_index* ix) {
 
 F64Scan f64_view(const fuelg_index* ix) {
   F64Scan x;
+  x.screen = ix->screen;
   x.X = ix->X64;
   x.n = ix->n;
   x.d = ix->d;
@@ -1179,6 +1183,10 @@ int fuelg_knn_f64(fuelg_index* ix, const double* queries, int64_t m, int32_t k, 
   OutBuf oi, od;
   FUELG_TRY(oi.init(out_idx, (size_t)m * k * sizeof(int64_t), s));
   FUELG_TRY(od.init(out_dist, (size_t)m * k * sizeof(double), s));
+  if (!ix->screen_tried && f64_screen_serves(ix->n, ix->d, m)) {
+    FUELG_TRY(f64_screen_build(ix->X64, ix->n, ix->d, s, &ix->screen));
+    ix->screen_tried = true;
+  }
   FUELG_TRY(f64_knn(f64_view(ix), Q, m, k, exclude_mode, static_cast<int64_t*>(oi.dptr),
                     static_cast<double*>(od.dptr), s));
   int64_t d2h = 0;

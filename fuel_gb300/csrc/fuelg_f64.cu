@@ -19,6 +19,12 @@
 // 23-30).  The keys below the threshold (fewer than kk <= 4096) are sorted in
 // shared memory.  Range lists are collected in index order and sorted stably
 // by distance.
+//
+// kNN rows of most shapes need FP64 for few pairs only: the FP32 tile scan over
+// rounded copies (F64Screen) keeps kk + margin candidates per query, their
+// distances are formed in fuel's f64 order, and a bound proves that no other
+// point can be among the kk nearest.  Queries without that proof take the
+// scan above, so results are the same bits.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -26,6 +32,7 @@
 #include <cub/device/device_segmented_sort.cuh>
 
 #include "../../include/fuelg.h"
+#include "fuelg_common.cuh"
 #include "fuelg_internal.h"
 
 namespace fuelg {
@@ -83,15 +90,16 @@ __device__ __forceinline__ uint64_t key64(double v) {
   return u == 0x8000000000000000ull ? 0ull : u;
 }
 
-// D[b, i] = distance(query q0 + b, point i) for the batch's rows.
+// D[b, i] = distance(query b of the batch, point i); rows: the batch's query
+// rows within Q, or nullptr for Q's rows in order.
 template <int ORDER>
 __global__ void __launch_bounds__(kT) dist64_kernel(const double* __restrict__ X, int64_t n, int d,
-                                                    const double* __restrict__ Q, int euclid,
-                                                    double* __restrict__ D) {
+                                                    const double* __restrict__ Q, const int32_t* __restrict__ rows,
+                                                    int euclid, double* __restrict__ D) {
   const int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x;
   if (i >= n) return;
   const int64_t b = blockIdx.y;
-  double v = sqdist64<ORDER>(Q + b * d, X + i * d, d);
+  double v = sqdist64<ORDER>(Q + (rows != nullptr ? rows[b] : b) * d, X + i * d, d);
   if (euclid) v = __dsqrt_rn(v);
   D[b * n + i] = v;
 }
@@ -225,7 +233,8 @@ __global__ void __launch_bounds__(kT) select64_kernel(const double* __restrict__
 // 485-488, 1163-1170, 1195-1216).  mode: FUELG_EXCLUDE_*; kk = min(k, n) for
 // NONE, min(k + 1, n) otherwise.
 __global__ void __launch_bounds__(kT) knn64_finish_kernel(const double* __restrict__ D, int64_t n, int kk, int k,
-                                                          int mode, int64_t q0, const uint64_t* __restrict__ thr,
+                                                          int mode, int64_t q0, const int32_t* __restrict__ rows,
+                                                          const uint64_t* __restrict__ thr,
                                                           const int64_t* __restrict__ n_less, int P,
                                                           int64_t* __restrict__ out_idx,
                                                           double* __restrict__ out_dist) {
@@ -266,7 +275,7 @@ __global__ void __launch_bounds__(kT) knn64_finish_kernel(const double* __restri
   if (mode == FUELG_EXCLUDE_LINEAR && kk > k) L = sk[k] == sk[k - 1] ? k + 1 : k;
   if (threadIdx.x == 0) s_self = -1;
   __syncthreads();
-  const int64_t self = q0 + b;
+  const int64_t self = rows != nullptr ? rows[b] : q0 + b;  // query row = output row
   if (mode != FUELG_EXCLUDE_NONE)
     for (int j = threadIdx.x; j < L; j += kT)
       if ((int64_t)si[j] == self) s_self = j;
@@ -275,8 +284,147 @@ __global__ void __launch_bounds__(kT) knn64_finish_kernel(const double* __restri
   for (int j = threadIdx.x; j < k; j += kT) {
     const int src = j + (sp >= 0 && j >= sp ? 1 : 0);
     const bool have = src < L;
-    out_idx[b * k + j] = have ? (int64_t)si[src] : -1;
-    out_dist[b * k + j] = have ? __longlong_as_double((long long)sk[src]) : __longlong_as_double(0x7ff0000000000000ll);
+    out_idx[self * k + j] = have ? (int64_t)si[src] : -1;
+    out_dist[self * k + j] =
+        have ? __longlong_as_double((long long)sk[src]) : __longlong_as_double(0x7ff0000000000000ll);
+  }
+}
+
+// ---- the FP32 screen ---------------------------------------------------------
+// Rows shifted by the index's first row (a common offset costs the rounded
+// copies no bits; coordinates that are not finite there shift by 0) and rounded
+// to f32.  err[r]: a bound on |row - copy| in the Euclidean norm; vint[r]: the
+// largest |value| of a copy whose values are all integers, else +inf.  all[0]:
+// the largest err (as bits of a double), all[1]: the largest vint (f32 bits).
+__global__ void __launch_bounds__(kT) narrow64_kernel(const double* __restrict__ X, int64_t rows, int d,
+                                                      const double* __restrict__ centre, float* __restrict__ out,
+                                                      double* __restrict__ err, float* __restrict__ vint,
+                                                      unsigned long long* __restrict__ all) {
+  const int lane = threadIdx.x & 31;
+  const int64_t step = (int64_t)gridDim.x * (kT / 32);
+  double worst = 0.0;
+  float vworst = 0.0f;
+  for (int64_t r = (int64_t)blockIdx.x * (kT / 32) + (threadIdx.x >> 5); r < rows; r += step) {
+    double e2 = 0.0;
+    float vm = 0.0f;
+    for (int c = lane; c < d; c += 32) {
+      const double c0 = centre[c];
+      const double v = isfinite(c0) ? X[r * d + c] - c0 : X[r * d + c];
+      const float f = __double2float_rn(v);
+      out[r * d + c] = f;
+      const double e = fabs(v - (double)f) + 1.2e-16 * fabs(v);  // and the shift's own rounding
+      e2 = fma(e, e, e2);
+      vm = f == rintf(f) && v == (double)f ? fmaxf(vm, fabsf(f)) : __int_as_float(0x7f800000);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      e2 += __shfl_xor_sync(kFull, e2, o);
+      vm = fmaxf(vm, __shfl_xor_sync(kFull, vm, o));
+    }
+    const double er = sqrt(e2) * (1.0 + 1e-12) + 1e-160;  // (squares below 1e-320 vanish)
+    if (lane == 0 && err != nullptr) {
+      err[r] = er;
+      vint[r] = vm;
+    }
+    worst = er > worst || er != er ? er : worst;  // a NaN stays
+    vworst = fmaxf(vworst, vm);
+  }
+  if (lane == 0 && all != nullptr) {
+    atomicMax(all, (unsigned long long)__double_as_longlong(worst));
+    atomicMax(all + 1, (unsigned long long)__float_as_uint(vworst));
+  }
+}
+
+// One warp per query: the f64 distances of the kk2 screened candidates, ranked by
+// (key, index), the exclude rule and the rows of knn64_finish_kernel; queries
+// without the proof are listed in redo instead.  Q, cand, qerr and qint start at
+// query q0, the outputs and the listed rows count from query 0.
+//
+// Proof: a point outside the list has a screened distance D >= D_last (f32, the
+// copies' distance times at most 1 + gamma), so its copies are at least
+// sqrt(D_last (1 - gamma)) apart and it is at least that less the two rounding
+// errors from the query; its f64 distance, computed with relative error g64, must
+// exceed the kk-th candidate's.  Where every value is an integer and every partial
+// sum below 2^24, the screened distances are exact and the list is final.
+template <int ORDER>
+__global__ void __launch_bounds__(kT) rescore64_kernel(const double* __restrict__ X, const double* __restrict__ Q,
+                                                       int64_t m, int64_t q0, int64_t n, int d,
+                                                       const uint64_t* __restrict__ cand, int kk2, int kk, int k, int mode, int euclid,
+                                                       const double* __restrict__ qerr,
+                                                       const float* __restrict__ qint, double xerr, float xint,
+                                                       int64_t* __restrict__ out_idx, double* __restrict__ out_dist,
+                                                       int32_t* __restrict__ redo, int32_t* __restrict__ nredo) {
+  extern __shared__ __align__(16) unsigned char smem64[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t* key = reinterpret_cast<uint64_t*>(smem64) + (size_t)warp * 2 * kk2;  // as found, then sorted
+  uint64_t* skey = key + kk2;
+  uint32_t* idx = reinterpret_cast<uint32_t*>(smem64 + (size_t)(kT / 32) * 16 * kk2) + (size_t)warp * 2 * kk2;
+  uint32_t* sidx = idx + kk2;
+  const int64_t q = (int64_t)blockIdx.x * (kT / 32) + warp;
+  if (q >= m) return;
+  const uint64_t* cq = cand + q * kk2;
+  const double* qr = Q + q * d;
+  for (int j = lane; j < kk2; j += 32) {
+    const uint64_t c = cq[j];
+    uint64_t kj = ~0ull;
+    uint32_t ij = 0xffffffffu;
+    // (an aborted screen leaves keys that name no row: they count as none)
+    if (c != KEY_NONE && (int64_t)key_idx(c) < n) {
+      ij = key_idx(c);
+      double v = sqdist64<ORDER>(qr, X + (int64_t)ij * d, d);
+      if (euclid) v = __dsqrt_rn(v);
+      kj = key64(v);
+    }
+    key[j] = kj;
+    idx[j] = ij;
+  }
+  __syncwarp();
+  int valid = 0;
+  for (int j = lane; j < kk2; j += 32) {
+    const uint64_t kj = key[j];
+    const uint32_t ij = idx[j];
+    if (ij == 0xffffffffu) continue;
+    valid++;
+    int rank = 0;
+    for (int i = 0; i < kk2; i++) rank += key[i] < kj || (key[i] == kj && idx[i] < ij) ? 1 : 0;
+    skey[rank] = kj;
+    sidx[rank] = ij;
+  }
+  valid = __reduce_add_sync(kFull, valid);
+  __syncwarp();
+  bool ok = valid >= kk;
+  if (ok && n > kk2) {  // otherwise every point was a candidate
+    const float qi = qint[q];
+    const double span = (double)qi + (double)xint;
+    if (!(span * span * d <= 16777216.0)) {
+      const double last = (double)key_dist(cq[kk2 - 1]);
+      const double gamma = (d + 8) * 0x1p-24 * 1.01, g64 = (d + 8) * 0x1p-53 * 1.01;
+      const double r = sqrt(fmax(0.0, last * (1.0 - gamma) - d * 0x1p-146)) * (1.0 - 1e-15) - (qerr[q] + xerr);
+      double low = r * r * (1.0 - g64 - 1e-15);
+      const double kth = __longlong_as_double((long long)skey[kk - 1]);
+      ok = r > 0.0 && low > 1e-280 && last < 3e38;
+      if (euclid) low = sqrt(low) * (1.0 - 1e-15);
+      ok = ok && kth < low;
+    }
+  }
+  if (!ok) {
+    if (lane == 0) redo[atomicAdd(nredo, 1)] = (int32_t)(q0 + q);
+    return;
+  }
+  int L = kk;
+  if (mode == FUELG_EXCLUDE_LINEAR && kk > k) L = skey[k] == skey[k - 1] ? k + 1 : k;
+  int sp = 0x7fffffff;
+  if (mode != FUELG_EXCLUDE_NONE)
+    for (int j = lane; j < L; j += 32)
+      if ((int64_t)sidx[j] == q0 + q) sp = j;
+  sp = __reduce_min_sync(kFull, sp);
+  out_idx += (q0 + q) * k;
+  out_dist += (q0 + q) * k;
+  for (int j = lane; j < k; j += 32) {
+    const int src = j + (j >= sp ? 1 : 0);
+    const bool have = src < L;
+    out_idx[j] = have ? (int64_t)sidx[src] : -1;
+    out_dist[j] = have ? __longlong_as_double((long long)skey[src]) : __longlong_as_double(0x7ff0000000000000ll);
   }
 }
 
@@ -424,13 +572,13 @@ int64_t batch_rows(int64_t n, int64_t m) {
   return std::min<int64_t>(B, 65535);
 }
 
-int launch_dist(const F64Scan& x, const double* Q, int64_t B, double* D, cudaStream_t s) {
+int launch_dist(const F64Scan& x, const double* Q, const int32_t* rows, int64_t B, double* D, cudaStream_t s) {
   const dim3 grid((unsigned)((x.n + kT - 1) / kT), (unsigned)B);
   const int euclid = x.metric == FUELG_METRIC_EUCLIDEAN ? 1 : 0;
   if (x.order == FUELG_ORDER_X86)
-    dist64_kernel<FUELG_ORDER_X86><<<grid, kT, 0, s>>>(x.X, x.n, x.d, Q, euclid, D);
+    dist64_kernel<FUELG_ORDER_X86><<<grid, kT, 0, s>>>(x.X, x.n, x.d, Q, rows, euclid, D);
   else
-    dist64_kernel<FUELG_ORDER_ARM><<<grid, kT, 0, s>>>(x.X, x.n, x.d, Q, euclid, D);
+    dist64_kernel<FUELG_ORDER_ARM><<<grid, kT, 0, s>>>(x.X, x.n, x.d, Q, rows, euclid, D);
   note_launch();
   FUELG_CUDA(cudaGetLastError());
   return ST_OK;
@@ -440,6 +588,95 @@ int allow_sort_smem() {
   const int bytes = kMaxSortKeys * (int)(sizeof(uint64_t) + sizeof(uint32_t));
   FUELG_CUDA(cudaFuncSetAttribute(knn64_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   FUELG_CUDA(cudaFuncSetAttribute(ties64_gather_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  return ST_OK;
+}
+
+}  // namespace
+
+// The rounded copy of a float64 index for the FP32 screen.
+struct F64Screen {
+  float* Xf = nullptr;  // [n, d]
+  double err = 0.0;     // bound on any row's |row - copy|
+  float vint = 0.0f;    // largest |value| when every copy value is an integer, else +inf
+};
+
+void f64_screen_free(F64Screen* f) {
+  if (!f) return;
+  if (f->Xf) cudaFree(f->Xf);
+  delete f;
+}
+
+// The screen's launches cost about 40 us more than the FP64 scan's, which a few
+// pairs do not repay.  Measured (us a call, FP64 scan / screen, k = 10): one
+// query, d = 16: n = 5000 59 / 82, 10 000 75 / 85, 20 000 104 / 84, 10^5 525 / 94;
+// m = 100, n = 2000, d = 16: 78 / 108, m = 300: 126 / 111; m = n = 1000, d = 2:
+// 102 / 104, d = 8: 135 / 106; m = n = 20 000, d = 16: 53 800 / 1210.
+bool f64_screen_serves(int64_t n, int d, int64_t m) {
+  return n >= 1000 && n < (1ll << 31) && tile_scan_supported(d, 1) &&
+         (n >= 16384 || (double)m * n * d >= 8e6);
+}
+
+int f64_screen_build(const double* X, int64_t n, int d, cudaStream_t s, F64Screen** out) {
+  *out = nullptr;
+  F64Screen* f = new F64Screen();
+  struct Guard {
+    F64Screen*& f;
+    ~Guard() { f64_screen_free(f); }
+  } guard{f};
+  if (cudaMalloc(&f->Xf, sizeof(float) * (size_t)n * d) != cudaSuccess) {
+    cudaGetLastError();
+    f->Xf = nullptr;
+    return ST_OK;  // no room for the copy: the FP64 scan answers
+  }
+  Scratch all;
+  FUELG_TRY(all.alloc(2 * sizeof(unsigned long long), s));
+  FUELG_CUDA(cudaMemsetAsync(all.p, 0, 2 * sizeof(unsigned long long), s));
+  narrow64_kernel<<<(unsigned)std::min<int64_t>((n + 7) / 8, 152 * 8), kT, 0, s>>>(
+      X, n, d, X, f->Xf, nullptr, nullptr, all.as<unsigned long long>());
+  note_launch();
+  FUELG_CUDA(cudaGetLastError());
+  unsigned long long h[2];
+  FUELG_CUDA(cudaMemcpyAsync(h, all.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+  FUELG_CUDA(cudaStreamSynchronize(s));
+  memcpy(&f->err, &h[0], sizeof(double));
+  const uint32_t vb = (uint32_t)h[1];
+  memcpy(&f->vint, &vb, sizeof(float));
+  if (!(f->err < 1e300)) return ST_OK;  // values outside the f32 range, NaN: no screen
+  *out = f;
+  f = nullptr;
+  return ST_OK;
+}
+
+namespace {
+
+// The FP64 scan of B-row batches: all m queries, or the `count` listed rows.
+int f64_knn_scan(const F64Scan& x, const double* Q, int64_t m, const int32_t* rows, int64_t kk, int k, int mode,
+                 int64_t* out_idx, double* out_dist, cudaStream_t s) {
+  FUELG_TRY(allow_sort_smem());
+  const int64_t B = batch_rows(x.n, m);
+  const int P = pow2_at_least(kk);
+  const size_t smem = (size_t)P * (sizeof(uint64_t) + sizeof(uint32_t));
+  Scratch D, thr, nl, ne;
+  FUELG_TRY(D.alloc(sizeof(double) * (size_t)B * x.n, s));
+  FUELG_TRY(thr.alloc(sizeof(uint64_t) * B, s));
+  FUELG_TRY(nl.alloc(sizeof(int64_t) * B, s));
+  FUELG_TRY(ne.alloc(sizeof(int64_t) * B, s));
+  for (int64_t q0 = 0; q0 < m; q0 += B) {
+    if (cancel_requested()) {
+      set_error("cancelled");
+      return ST_ECANCELLED;
+    }
+    const int64_t Bb = std::min<int64_t>(B, m - q0);
+    const int32_t* rb = rows != nullptr ? rows + q0 : nullptr;
+    FUELG_TRY(launch_dist(x, rows != nullptr ? Q : Q + q0 * x.d, rb, Bb, D.as<double>(), s));
+    select64_kernel<<<(unsigned)Bb, kT, 0, s>>>(D.as<double>(), x.n, kk, thr.as<uint64_t>(), nl.as<int64_t>(),
+                                                ne.as<int64_t>());
+    note_launch();
+    knn64_finish_kernel<<<(unsigned)Bb, kT, smem, s>>>(D.as<double>(), x.n, (int)kk, k, mode, q0, rb,
+                                                       thr.as<uint64_t>(), nl.as<int64_t>(), P, out_idx, out_dist);
+    note_launch();
+    FUELG_CUDA(cudaGetLastError());
+  }
   return ST_OK;
 }
 
@@ -457,30 +694,57 @@ int f64_knn(const F64Scan& x, const double* Q, int64_t m, int k, int mode, int64
     FUELG_CUDA(cudaGetLastError());
     return ST_OK;
   }
-  FUELG_TRY(allow_sort_smem());
-  const int64_t B = batch_rows(x.n, m);
-  const int P = pow2_at_least(kk);
-  const size_t smem = (size_t)P * (sizeof(uint64_t) + sizeof(uint32_t));
-  Scratch D, thr, nl, ne;
-  FUELG_TRY(D.alloc(sizeof(double) * (size_t)B * x.n, s));
-  FUELG_TRY(thr.alloc(sizeof(uint64_t) * B, s));
-  FUELG_TRY(nl.alloc(sizeof(int64_t) * B, s));
-  FUELG_TRY(ne.alloc(sizeof(int64_t) * B, s));
-  for (int64_t q0 = 0; q0 < m; q0 += B) {
-    if (cancel_requested()) {
+  // candidates kept beyond kk: ranks for the proof's error bound to fall between
+  // (kk <= 28 then still fits the tile scan's sorted lists of 32)
+  const int64_t kk2 = kk + std::max<int64_t>(4, kk / 8);
+  if (x.screen == nullptr || !f64_screen_serves(x.n, x.d, m) ||
+      !tile_scan_supported(x.d, (int)std::min<int64_t>(kk2, 1 << 20)) || m >= (1ll << 31))
+    return f64_knn_scan(x, Q, m, nullptr, kk, k, mode, out_idx, out_dist, s);
+  // query batches: their copies, candidates and redo lists stay below ~1 GiB
+  const int64_t mb = std::min<int64_t>(m, std::max<int64_t>(64, (1ll << 30) / (8 * kk2 + 4 * x.d + 16)));
+  Scratch qf, qerr, qint, cand, redo, words;
+  FUELG_TRY(qf.alloc(sizeof(float) * (size_t)mb * x.d, s));
+  FUELG_TRY(qerr.alloc(sizeof(double) * mb, s));
+  FUELG_TRY(qint.alloc(sizeof(float) * mb, s));
+  FUELG_TRY(cand.alloc(sizeof(uint64_t) * (size_t)mb * kk2, s));
+  FUELG_TRY(redo.alloc(sizeof(int32_t) * mb, s));
+  FUELG_TRY(words.alloc(2 * sizeof(int32_t), s));  // redo count, device status
+  const size_t smem = (size_t)(kT / 32) * 2 * kk2 * (sizeof(uint64_t) + sizeof(uint32_t));
+  auto rescore = x.order == FUELG_ORDER_X86 ? rescore64_kernel<FUELG_ORDER_X86> : rescore64_kernel<FUELG_ORDER_ARM>;
+  FUELG_CUDA(cudaFuncSetAttribute(rescore, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
+  for (int64_t q0 = 0; q0 < m; q0 += mb) {
+    const int64_t mc = std::min<int64_t>(mb, m - q0);
+    const double* Qb = Q + q0 * x.d;
+    FUELG_CUDA(cudaMemsetAsync(words.p, 0, 2 * sizeof(int32_t), s));
+    narrow64_kernel<<<(unsigned)std::min<int64_t>((mc + 7) / 8, 152 * 8), kT, 0, s>>>(
+        Qb, mc, x.d, x.X, qf.as<float>(), qerr.as<double>(), qint.as<float>(), nullptr);
+    note_launch();
+    ExactScanParams p;
+    p.A = qf.as<float>();
+    p.m = mc;
+    p.B = x.screen->Xf;
+    p.n = x.n;
+    p.d = x.d;
+    p.kind = KIND_KNN;
+    p.order = ORDER_X86;  // fewer operations; any f32 order is within the bound
+    p.metric = METRIC_SQEUCLIDEAN;
+    p.kk = (int)kk2;
+    FUELG_TRY(tile_scan_topk(p, cand.as<uint64_t>(), words.as<int>() + 1, s));
+    rescore<<<(unsigned)((mc + kT / 32 - 1) / (kT / 32)), kT, smem, s>>>(
+        x.X, Qb, mc, q0, x.n, x.d, cand.as<uint64_t>(), (int)kk2, (int)kk, k, mode,
+        x.metric == FUELG_METRIC_EUCLIDEAN ? 1 : 0, qerr.as<double>(), qint.as<float>(), x.screen->err,
+        x.screen->vint, out_idx, out_dist, redo.as<int32_t>(), words.as<int32_t>());
+    note_launch();
+    FUELG_CUDA(cudaGetLastError());
+    int32_t h[2];
+    FUELG_CUDA(cudaMemcpyAsync(h, words.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+    FUELG_CUDA(cudaStreamSynchronize(s));
+    if ((h[1] & DEV_CANCELLED) || cancel_requested()) {
       set_error("cancelled");
       return ST_ECANCELLED;
     }
-    const int64_t Bb = std::min<int64_t>(B, m - q0);
-    FUELG_TRY(launch_dist(x, Q + q0 * x.d, Bb, D.as<double>(), s));
-    select64_kernel<<<(unsigned)Bb, kT, 0, s>>>(D.as<double>(), x.n, kk, thr.as<uint64_t>(), nl.as<int64_t>(),
-                                                ne.as<int64_t>());
-    note_launch();
-    knn64_finish_kernel<<<(unsigned)Bb, kT, smem, s>>>(D.as<double>(), x.n, (int)kk, k, mode, q0,
-                                                       thr.as<uint64_t>(), nl.as<int64_t>(), P,
-                                                       out_idx + q0 * k, out_dist + q0 * k);
-    note_launch();
-    FUELG_CUDA(cudaGetLastError());
+    if (h[0] > 0)
+      FUELG_TRY(f64_knn_scan(x, Q, h[0], redo.as<int32_t>(), kk, k, mode, out_idx, out_dist, s));
   }
   return ST_OK;
 }
@@ -512,7 +776,7 @@ int f64_lists(const F64Scan& x, const double* Q, int64_t m, bool range, int64_t 
       return ST_ECANCELLED;
     }
     const int64_t Bb = std::min<int64_t>(B, m - q0);
-    FUELG_TRY(launch_dist(x, Q + q0 * x.d, Bb, D.as<double>(), s));
+    FUELG_TRY(launch_dist(x, Q + q0 * x.d, nullptr, Bb, D.as<double>(), s));
     if (range) {
       range_count64_kernel<<<(unsigned)Bb, kT, 0, s>>>(D.as<double>(), x.n, q0, drop_self ? 1 : 0, radius,
                                                        cnt.as<int64_t>());
