@@ -51,13 +51,6 @@ constexpr int kTileLogCap = 32 * kSel - kTileP;
 constexpr int kTileSmemMax =
     (int)sizeof(float) * kTileMaxD * (kTileQS + 2 * kTilePS);  // 167 KB
 
-// One key into the warp's ascending list of 32 (the largest falls out).
-__device__ __forceinline__ uint64_t warp_insert32(uint64_t kept, uint64_t key, int lane) {
-  const uint64_t up = ((uint64_t)__shfl_up_sync(0xffffffffu, (uint32_t)(kept >> 32), 1) << 32) |
-                      __shfl_up_sync(0xffffffffu, (uint32_t)kept, 1);
-  return kept < key ? kept : (lane == 0 || up < key) ? key : up;
-}
-
 // SMALL: kk <= 32, each row's keys as a sorted list in shared memory that every
 // passing key enters at once (the limit is never stale, so the fewest tiles
 // take the slow path); otherwise kept keys and an append log in global memory.

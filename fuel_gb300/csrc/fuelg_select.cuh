@@ -105,6 +105,41 @@ static __device__ __noinline__ uint64_t warp_select(const uint64_t* __restrict__
   return total >= kk ? kth : KEY_NONE;
 }
 
+// A distance-word limit t for the keys the lanes hold in hi[] (0xffffffff: no
+// key): at least kk of them lie below t, and no more than kk + slack unless more
+// share one word.  Returns t, the number below it in *below.  total >= kk keys,
+// words in [hmin, hmax].  Where the words are spread evenly, aiming at the rank
+// between the two counts takes two or three steps; every third step halves the
+// range instead, which bounds them.
+template <int N>
+__device__ __forceinline__ uint32_t warp_cut(const uint32_t (&hi)[N], int total, int kk, int slack, uint32_t hmin,
+                                             uint32_t hmax, int* below) {
+  uint32_t lo = hmin, up = hmax + 1;  // count(< lo) = clo < kk <= cnt = count(< up)
+  int clo = 0, cnt = total;
+#pragma unroll 1
+  for (int step = 1; cnt > kk + slack && up - lo > 1; step++) {
+    const uint32_t span = up - lo;
+    uint32_t mid = lo + span / 2;
+    if (step % 3 != 0) {
+      const float f = ((float)(kk - clo) + 0.5f * (float)slack) / (float)(cnt - clo);
+      mid = lo + min(span - 1, max(1u, (uint32_t)(f * (float)span)));
+    }
+    int c = 0;
+#pragma unroll
+    for (int i = 0; i < N; i++) c += hi[i] < mid ? 1 : 0;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (c >= kk) {
+      up = mid;
+      cnt = c;
+    } else {
+      lo = mid;
+      clo = c;
+    }
+  }
+  *below = cnt;
+  return up;
+}
+
 // v of the lanes sorted ascending over the warp (bitonic network, 15 stages).
 __device__ __forceinline__ uint64_t warp_sort32(uint64_t v, int lane) {
 #pragma unroll
@@ -135,6 +170,13 @@ __device__ __forceinline__ uint64_t warp_merge32(uint64_t kept, uint64_t v, int 
     kept = (o < kept) == ((lane & j) == 0) ? o : kept;
   }
   return kept;
+}
+
+// One key into the warp's ascending list of 32 (the largest falls out).
+__device__ __forceinline__ uint64_t warp_insert32(uint64_t kept, uint64_t key, int lane) {
+  const uint64_t up = ((uint64_t)__shfl_up_sync(0xffffffffu, (uint32_t)(kept >> 32), 1) << 32) |
+                      __shfl_up_sync(0xffffffffu, (uint32_t)kept, 1);
+  return kept < key ? kept : (lane == 0 || up < key) ? key : up;
 }
 
 __device__ __forceinline__ uint64_t shfl_u64(uint64_t v, int src) {

@@ -42,6 +42,25 @@ int make_map_bf16(CUtensorMap* tm, const void* ptr, int64_t rows, int dp, int bo
   return ST_OK;
 }
 
+int make_map_norm(CUtensorMap* tm, const void* ptr, int64_t rows, int box_rows) {
+  auto fn = encode_fn();
+  if (!fn) {
+    set_error("cuTensorMapEncodeTiled is unavailable from the driver");
+    return ST_ECUDA;
+  }
+  cuuint64_t dims[2] = {16, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {32};
+  cuuint32_t box[2] = {16, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (%d) for the norm operand of %lld rows", (int)r, (long long)rows);
+    return ST_ECUDA;
+  }
+  return ST_OK;
+}
 
 }  // namespace tcx
 }  // namespace fuelg
