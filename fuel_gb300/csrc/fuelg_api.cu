@@ -1026,8 +1026,9 @@ int fuelg_range(fuelg_index* ix, const float* queries, int64_t m, double radius,
   p.metric = ix->metric;
   fuelg_range_result* r = new fuelg_range_result();
   r->m = m;
+  int passes = 0;
   int st = exact_range(p, (float)radius, exclude_self ? 1 : 0, &r->off, &r->idx, &r->dist, &r->total,
-                       dstat.as<int>(), s);
+                       dstat.as<int>(), s, nullptr, &passes);
   if (st == ST_OK) st = read_dev_status(dstat.as<int>(), s);
   const double ms = tm.stop();
   if (st != ST_OK) {
@@ -1037,7 +1038,7 @@ int fuelg_range(fuelg_index* ix, const float* queries, int64_t m, double radius,
   if (stats) {
     stats->device_ms = ms;
     stats->h2d_bytes = q.h2d;
-    stats->distance_evals = 2 * m * ix->n;
+    stats->distance_evals = passes * m * ix->n;
     stats->precision_used = FUELG_PREC_FP32;
     meter.fill(stats);
   }

@@ -303,8 +303,18 @@ int pairwise_launch(const float* X, int64_t n, int d, int metric, int order, int
 
 // Range search, CSR output on the device.  Allocates *off/*idx/*dist with cudaMalloc.
 // radii (device, p.m entries, or nullptr): a radius per query row instead of `radius`.
+// *passes: how often every distance was formed.
 int exact_range(const ExactScanParams& p, float radius, int exclude_self, int64_t** d_off, int64_t** d_idx,
-                float** d_dist, int64_t* total, int* dev_status, cudaStream_t stream, const float* radii = nullptr);
+                float** d_dist, int64_t* total, int* dev_status, cudaStream_t stream, const float* radii = nullptr,
+                int* passes = nullptr);
+
+// The same in register tiles (fuelg_range.cu), d_off [p.m + 1] given: one pass, the
+// hits of a query sorted from its slots.
+bool tile_range_supported(int d);
+int tile_range(const ExactScanParams& p, float radius, int exclude_self, int64_t* d_off, int64_t** d_idx,
+               float** d_dist, int64_t* total, cudaStream_t stream, const float* radii, int* passes);
+// (distance, index) keys into an index and a distance array.
+int split_keys(const uint64_t* keys, int64_t total, int64_t* idx, float* dist, cudaStream_t stream);
 
 // -------- tie-inclusive kNN lists (fuelg_ties.cu) ------------------------------
 // Keys kept per query for tie-inclusive lists of kq neighbours (kq plus spare ranks).

@@ -741,9 +741,10 @@ int exact_knn_in_scratch(const ExactScanParams& p, int k, int exclude_mode, int6
 }
 
 // ---------------------------------------------------------------------------
-// Range search (linear_scan_range, src/api/search.rs:154-166): two passes of
-// the same scan -- count, then fill at scanned offsets -- then a segmented
-// sort of the (distance, index) keys of every query.
+// Range search (linear_scan_range, src/api/search.rs:154-166) of rows of more than
+// 128 dimensions (fuelg_range.cu has the others): two passes of the same scan --
+// count, then fill at scanned offsets -- then a segmented sort of the (distance,
+// index) keys of every query.
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -829,9 +830,19 @@ int launch_range(const ScanArgs& a, const Plan& pl, int64_t qblocks, float radiu
 
 }  // namespace
 
+int split_keys(const uint64_t* keys, int64_t total, int64_t* idx, float* dist, cudaStream_t stream) {
+  split_keys_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(keys, total, idx, dist);
+  ::fuelg::note_launch();
+  FUELG_CUDA(cudaGetLastError());
+  return ST_OK;
+}
+
 int exact_range(const ExactScanParams& p, float radius, int exclude_self, int64_t** d_off, int64_t** d_idx,
-                float** d_dist, int64_t* total, int* dev_status, cudaStream_t stream, const float* radii) {
+                float** d_dist, int64_t* total, int* dev_status, cudaStream_t stream, const float* radii, int* passes) {
   (void)dev_status;
+  int unused = 0;
+  if (passes == nullptr) passes = &unused;
+  *passes = 0;
   *d_off = nullptr;
   *d_idx = nullptr;
   *d_dist = nullptr;
@@ -841,6 +852,8 @@ int exact_range(const ExactScanParams& p, float radius, int exclude_self, int64_
     FUELG_CUDA(cudaMemsetAsync(*d_off, 0, sizeof(int64_t) * (p.m + 1), stream));
     return ST_OK;
   }
+  if (p.kind == KIND_KNN && tile_range_supported(p.d))
+    return tile_range(p, radius, exclude_self, *d_off, d_idx, d_dist, total, stream, radii, passes);
   Plan pl;
   FUELG_TRY(make_plan(p, true, scan_np(p.kind, p.order), &pl));
   const int S = pl.S_grid * pl.ws;
@@ -879,6 +892,7 @@ int exact_range(const ExactScanParams& p, float radius, int exclude_self, int64_
                                                    offs, out, fill, stream);
   };
   FUELG_TRY(run(false, nullptr, nullptr));
+  *passes = 1;
   size_t tb = 0;
   FUELG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, counts.as<int64_t>(), scanned.as<int64_t>(), mS + 1, stream));
   FUELG_TRY(tmp.alloc(tb, stream));
@@ -893,6 +907,7 @@ int exact_range(const ExactScanParams& p, float radius, int exclude_self, int64_
   FUELG_TRY(keys.alloc(sizeof(uint64_t) * tot, stream));
   FUELG_TRY(keys_sorted.alloc(sizeof(uint64_t) * tot, stream));
   FUELG_TRY(run(true, scanned.as<int64_t>(), keys.as<uint64_t>()));
+  *passes = 2;
   size_t sb = 0;
   FUELG_CUDA(cub::DeviceSegmentedSort::SortKeys(nullptr, sb, keys.as<uint64_t>(), keys_sorted.as<uint64_t>(), tot,
                                                 p.m, *d_off, *d_off + 1, stream));
@@ -902,10 +917,7 @@ int exact_range(const ExactScanParams& p, float radius, int exclude_self, int64_
                                                 p.m, *d_off, *d_off + 1, stream));
   FUELG_CUDA(cudaMalloc(d_idx, sizeof(int64_t) * tot));
   FUELG_CUDA(cudaMalloc(d_dist, sizeof(float) * tot));
-  split_keys_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(keys_sorted.as<uint64_t>(), tot, *d_idx,
-                                                                       *d_dist); ::fuelg::note_launch();
-  FUELG_CUDA(cudaGetLastError());
-  return ST_OK;
+  return split_keys(keys_sorted.as<uint64_t>(), tot, *d_idx, *d_dist, stream);
 }
 
 }  // namespace fuelg

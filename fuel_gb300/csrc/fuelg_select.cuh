@@ -184,4 +184,37 @@ __device__ __forceinline__ uint64_t shfl_u64(uint64_t v, int src) {
          __shfl_sync(0xffffffffu, (uint32_t)v, src);
 }
 
+// Ascending bitonic sort of the warp's 32 R keys, element e = lane * R + r in v[r].
+template <int R>
+__device__ __forceinline__ void warp_sort_keys(uint64_t (&v)[R], int lane) {
+#pragma unroll
+  for (int k2 = 2; k2 <= 32 * R; k2 <<= 1) {
+#pragma unroll
+    for (int j = k2 >> 1; j > 0; j >>= 1) {
+      if (j >= R) {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          const uint64_t o = ((uint64_t)__shfl_xor_sync(0xffffffffu, (uint32_t)(v[r] >> 32), j / R) << 32) |
+                             __shfl_xor_sync(0xffffffffu, (uint32_t)v[r], j / R);
+          const int e = lane * R + r;
+          const bool up = (e & k2) == 0;
+          const bool lower = (e & j) == 0;
+          v[r] = (lower == up) ? (o < v[r] ? o : v[r]) : (o > v[r] ? o : v[r]);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          if (r & j) continue;
+          const int e = lane * R + r;
+          const bool up = (e & k2) == 0;
+          const uint64_t x = v[r], y = v[r ^ j];
+          const bool sw = up ? (x > y) : (x < y);
+          v[r] = sw ? y : x;
+          v[r ^ j] = sw ? x : y;
+        }
+      }
+    }
+  }
+}
+
 }  // namespace fuelg
