@@ -32,6 +32,7 @@
 #include "fuelg_exact.cuh"
 #include "fuelg_internal.h"
 #include "fuelg_tc_common.cuh"
+#include "fuelg_tile.cuh"
 
 namespace fuelg {
 namespace {
@@ -397,24 +398,37 @@ __device__ __forceinline__ float norm2_blocked(F v, int d) {
 }
 
 // Warp-specialised persistent screen over a list of 128-row items:
-//   warps 0-3  loaders: thread 0 copies the NEXT item's rows (contiguous in
-//              memory) into one of two staging buffers with one bulk copy; all
-//              128 convert the current item's rows from staging into BF16 hi /
-//              lo (SW128) and |x|^2, one row per thread, into one of two A
-//              buffers; on a problem change they stage the problem's centres
-//              (hi / lo, SW128), norms and parameters
-//   warp 4     TMEM owner; lane 0 issues the three products per K step
-//              (x_hi c_hi + x_hi c_lo + x_lo c_hi) into one of two 256-column
-//              accumulators and commits
-//   warps 5-8  epilogue: screen, labels, sums of changed rows
+//   warps 0-7   loaders: convert the current item's rows from one of two staging
+//               buffers into BF16 hi / lo (SW128) and |x|^2 into one of two A
+//               buffers; on a problem change they stage the problem's centres
+//               (hi / lo, SW128), norms and parameters
+//   warp 8      TMEM owner; one lane issues the three products per K step
+//               (x_hi c_hi + x_hi c_lo + x_lo c_hi) into one of two 256-column
+//               accumulators and commits, and copies the rows of the item after
+//               next (contiguous in memory) into the staging buffer just converted
+//               with one bulk copy
+//   warps 9-16  epilogue, four warps per accumulator: screen, labels, sums of
+//               changed rows
 // so the row copy of item t+1, its conversion, the MMAs and the epilogue of
-// item t overlap.  Barriers: stage_full[s] (bulk copy bytes), a_full[b] (128
-// loader arrivals), acc_full[b] (the MMA commit), item_done[b] (128 epilogue
-// arrivals: A[b], TMEM[b] and the item's parameters are free again).  On a
-// problem change the loaders first wait for the previous item to retire, so
+// item t overlap.  Barriers: stage_full[s] (bulk copy bytes), a_full[b] (eight
+// loader warps), acc_full[b] (the MMA commit: A[b] is free again),
+// item_done[b] (four epilogue warps: TMEM[b] is free again).  An item's
+// parameters and row norms have one of four places: item t's are written after
+// the MMAs of item t-2, which were issued after item t-4 retired.  On a
+// problem change the loaders first wait for both previous items to retire, so
 // the single centre buffer is never replaced under a reader.  Every wait is
 // bounded.
-constexpr int kTcThreads = 288;
+//
+// Bound by the latency of 17 warps that each depend on few others (1.5 instructions
+// a cycle, tensor pipe 4 %).  Screens of 76 900 items (9.8 million rows of 32 or 64
+// dimensions, k to 256): 2.38 ms with one group of four epilogue warps that branched
+// per column (123 cycles a column) and four loader warps with one row per thread;
+// 1.29 now.  On the way: branch-free passes and two groups 1.9, packed steps and the
+// problem looked up at a change only 1.75, CTA ranges by the new costs 1.29.  The
+// issuer's role on an epilogue warp (16 warps) spilled and was 15 % slower, as was
+// holding the screen values of up to 32 columns between the passes (5 %).
+constexpr int kTcThreads = 544;
+constexpr int kTcLoaders = 256;
 constexpr uint32_t kTcA = 32768;   // one A buffer: hi 16 KB + lo 16 KB
 constexpr uint32_t kTcB = 65536;   // the centre buffer: hi 32 KB + lo 32 KB (256 centres)
 constexpr uint32_t kTcS = 32768;   // one staging buffer: 128 rows x 64 f32
@@ -425,17 +439,17 @@ struct ItemMeta {  // one item's problem parameters, written by the loaders
   int32_t p, i0, kp, d, k, L, e_lo, cnt_off;
 };
 
-// + norms (2 x 256 floats), maxima (4), row norms (2 x 128), metadata (2), 9 mbarriers,
+// + norms (2 x 256 floats), maxima (4), row norms (4 x 128), metadata (4), 9 mbarriers,
 // TMEM address and abort word, 1 KB alignment
 constexpr size_t kTcSmem =
-    1024 + kTcSmall + 4 * 2 * 256 + 4 * 4 + 4 * 2 * 128 + sizeof(ItemMeta) * 2 + 8 * 9 + 8 + 64;
+    1024 + kTcSmall + 4 * 2 * 256 + 4 * 4 + 4 * 4 * 128 + sizeof(ItemMeta) * 4 + 8 * 9 + 8 + 64;
 
-// Every loader thread (warps 0-3, named barrier 1) learns whether all of
+// Every loader thread (warps 0-7, named barrier 1) learns whether all of
 // them passed `v`.
 __device__ __forceinline__ bool loaders_all(bool v) {
   uint32_t r;
   asm volatile(
-      "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.and.pred p, 1, 128, q;\n selp.u32 %0, 1, 0, p;\n}"
+      "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.and.pred p, 1, 256, q;\n selp.u32 %0, 1, 0, p;\n}"
       : "=r"(r)
       : "r"((uint32_t)v)
       : "memory");
@@ -454,10 +468,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
   unsigned char* sBl = sBh + kTcB / 2;
   float* cn2s = reinterpret_cast<float*>(base + kTcSmall);  // [256] |c|^2 of the staged problem
   float* cns = cn2s + 256;                                   // [256] |c|
-  float* cmaxs = cns + 256;                                  // [0] max |c|^2 (bits), spare
-  float* xn2s = cmaxs + 4;                                   // [2 buffers][128] |x|^2
-  ItemMeta* meta = reinterpret_cast<ItemMeta*>(xn2s + 2 * 128);
-  uint64_t* stage_full = reinterpret_cast<uint64_t*>(meta + 2);
+  float* cmaxs = cns + 256;                                  // max |c|^2, max |c| (bits)
+  float* xn2s = cmaxs + 4;                                   // [4 items][128] |x|^2
+  ItemMeta* meta = reinterpret_cast<ItemMeta*>(xn2s + 4 * 128);
+  uint64_t* stage_full = reinterpret_cast<uint64_t*>(meta + 4);
   uint64_t* a_full = stage_full + 2;
   uint64_t* acc_full = a_full + 2;
   uint64_t* item_done = acc_full + 2;
@@ -468,15 +482,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
   if (tid == 0) {
     for (int b = 0; b < 2; b++) {
       tcx::mbar_init(&stage_full[b], 1);
-      tcx::mbar_init(&a_full[b], kTcRows);
+      tcx::mbar_init(&a_full[b], kTcLoaders / 32);  // one arrival per warp
       tcx::mbar_init(&acc_full[b], 1);
-      tcx::mbar_init(&item_done[b], kTcRows);
+      tcx::mbar_init(&item_done[b], kTcRows / 32);
     }
     tcx::mbar_init(fin, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 4) {
+  if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tcx::smem_u32(tmem_holder)),
                  "r"(512)
                  : "memory");
@@ -509,55 +523,47 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
     return (uint32_t)(rows * pr.d * 4);
   };
 
-  if (warp < 4) {
+  if (warp < 8) {
     // ---- loaders ----------------------------------------------------------
-    int q = -1, cur_p = -1, qn = -1;
-    int issued[2] = {0, 0};  // copies (or plain arrivals) armed per staging buffer, thread 0
-    // the first item's rows
-    if (tid == 0 && nlt > 0) {
-      issued[0] = 1;
-      qn = problem_of(it0, -1);
-      const BProb pn = probs[ta.tcp[qn]];
-      const int64_t i0n = (it0 - ta.item_begin[qn]) * kTcRows;
-      const uint32_t by = bulk_bytes(pn, i0n);
-      if (by) {
-        tcx::mbar_expect_tx(&stage_full[0], by);
-        tcx::bulk_load(base + kTcOffS, X + pn.x_off + i0n * pn.d, by, &stage_full[0]);
-      } else {
-        tcx::mbar_arrive(&stage_full[0]);
-      }
-    }
+    int q = -1;
+    BProb pr;                            // the problem, looked up at a change only (three dependent loads)
+    int64_t q_begin = 0, q_end = 0;      // its items
+    int p = 0, kp = 0;
     for (int64_t lt = 0; lt < nlt; lt++) {
-      const int b = (int)(lt & 1);
+      const int b = (int)(lt & 1), slot = (int)(lt & 3);
       const uint32_t ph = (uint32_t)((lt >> 1) & 1);
-      // item lt-2 retired: its A buffer, accumulator and parameters are free.
-      // The loaders leave together (a vote on their named barrier), so the
-      // barriers below never wait for a loader that left.
-      bool ok = !*abort_flag && tcx::mbar_wait(&item_done[b], ph ^ 1u, abort_flag);
+      // the products of item lt-2 are made: its A buffer is free, and item lt-4
+      // has retired.  The loaders leave together (a vote on their named barrier),
+      // so the barriers below never wait for a loader that left.
+      bool ok = !*abort_flag && tcx::mbar_wait(&acc_full[b], ph ^ 1u, abort_flag);
       if (!ok && !*abort_flag) atomicOr(ta.status, DEV_TIMEOUT);
       if (!loaders_all(ok)) {
         *abort_flag = 1;
         break;
       }
       const int64_t item = it0 + lt;
-      q = problem_of(item, q);
-      const int p = ta.tcp[q];
-      const BProb pr = probs[p];
-      const int kp = (pr.k + 15) & ~15;
-      const int64_t i0 = (item - ta.item_begin[q]) * kTcRows;
-      if (p != cur_p) {
-        // a new problem: the previous item must retire before its centres go
+      if (item >= q_end) {
+        q = problem_of(item, q);
+        p = ta.tcp[q];
+        pr = probs[p];
+        q_begin = ta.item_begin[q];
+        q_end = ta.item_begin[q + 1];
+        kp = (pr.k + 15) & ~15;
+        // the previous items must retire before their centres go (a wait by parity is
+        // for the barrier's current phase: item lt-1's products come after item lt-3
+        // retired)
         if (lt > 0) {
-          const int pb = (int)((lt - 1) & 1);
-          ok = !*abort_flag && tcx::mbar_wait(&item_done[pb], (uint32_t)(((lt - 1) >> 1) & 1), abort_flag);
+          const uint32_t ph1 = (uint32_t)(((lt - 1) >> 1) & 1);
+          ok = !*abort_flag && tcx::mbar_wait(&acc_full[b ^ 1], ph1, abort_flag) &&
+               tcx::mbar_wait(&item_done[b ^ 1], ph1, abort_flag) &&
+               tcx::mbar_wait(&item_done[b], ph ^ 1u, abort_flag);
           if (!ok && !*abort_flag) atomicOr(ta.status, DEV_TIMEOUT);
           if (!loaders_all(ok)) {
             *abort_flag = 1;
             break;
           }
         }
-        cur_p = p;
-        for (int e = tid; e < kp * 8; e += kTcRows) {
+        for (int e = tid; e < kp * 8; e += kTcLoaders) {
           const int j = e >> 3, ch = e & 7;
           uint32_t hw[4], lw[4];
 #pragma unroll
@@ -575,10 +581,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
           *reinterpret_cast<uint4*>(sBh + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
           *reinterpret_cast<uint4*>(sBl + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
         }
-        if (tid == 0) cmaxs[0] = 0.0f;
-        asm volatile("bar.sync 1, %0;" ::"n"(kTcRows) : "memory");  // loaders only
+        if (tid == 0) cmaxs[0] = cmaxs[1] = 0.0f;
+        asm volatile("bar.sync 1, %0;" ::"n"(kTcLoaders) : "memory");  // loaders only
         float m2 = 0.0f;
-        for (int j = tid; j < 256; j += kTcRows) {
+        for (int j = tid; j < 256; j += kTcLoaders) {
           float v = 0.0f;
           if (j < pr.k) {
             const float* cj = C + pr.c_off + (int64_t)j * pr.d;
@@ -592,29 +598,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
         }
         // non-negative floats order like their bit patterns
         atomicMax(reinterpret_cast<int*>(cmaxs), __float_as_int(m2));
+        atomicMax(reinterpret_cast<int*>(cmaxs) + 1, __float_as_int(sqrtf(m2)));
       }
-      // the next item's rows into the other staging buffer: its previous
-      // contents (item lt-1) were converted before every loader passed the
-      // vote above
-      if (tid == 0 && lt + 1 < nlt) {
-        const int s = (int)((lt + 1) & 1);
-        issued[s]++;
-        qn = problem_of(item + 1, qn);
-        const BProb pn = probs[ta.tcp[qn]];
-        const int64_t i0n = (item + 1 - ta.item_begin[qn]) * kTcRows;
-        const uint32_t by = bulk_bytes(pn, i0n);
-        if (by) {
-          tcx::mbar_expect_tx(&stage_full[s], by);
-          tcx::bulk_load(base + kTcOffS + (uint32_t)s * kTcS, X + pn.x_off + i0n * pn.d, by, &stage_full[s]);
-        } else {
-          tcx::mbar_arrive(&stage_full[s]);
-        }
-      }
-      // this item's rows -> BF16 hi / lo (zero padded), FP32 norms; thread = row
+      const int64_t i0 = (item - q_begin) * kTcRows;
+      // this item's rows -> BF16 hi / lo (zero padded), FP32 norms: a thread takes
+      // chunks of 8 values, the 4 (d <= 32) or 8 chunks of a row on neighbouring
+      // lanes, so a warp reads and writes shared memory in runs
       unsigned char* sAh = base + (uint32_t)b * kTcA;
       unsigned char* sAl = sAh + kTcA / 2;
-      const int64_t i = i0 + tid;
-      const bool live = pr.active && i < pr.n;
       ok = !*abort_flag && tcx::mbar_wait(&stage_full[b], ph, abort_flag);
       if (!ok && !*abort_flag) atomicOr(ta.status, DEV_TIMEOUT);
       if (!loaders_all(ok)) {
@@ -622,45 +613,66 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
         break;
       }
       const bool bulk = bulk_bytes(pr, i0) != 0;
-      const float* srow = reinterpret_cast<const float*>(base + kTcOffS + (uint32_t)b * kTcS) + tid * pr.d;
-      const float* xr = X + pr.x_off + (live ? i : 0) * pr.d;
-      float pn[8];
-#pragma unroll
-      for (int l = 0; l < 8; l++) pn[l] = 0.0f;
-      // chunks of 8 values in a per-row rotated order (row t starts at chunk
-      // t & 7), so the staging reads of a warp spread over the banks; the
-      // norm keeps its 8 interleaved chains of ceil(d/8) terms and 3-level tree
-#pragma unroll 2
-      for (int jj = 0; jj < 8; jj++) {
-        const int j = (jj + tid) & 7;
-        float x[8];
-        if (live && bulk && 8 * j + 7 < pr.d) {
-          const float4 a4 = *reinterpret_cast<const float4*>(srow + 8 * j);
-          const float4 b4 = *reinterpret_cast<const float4*>(srow + 8 * j + 4);
-          x[0] = a4.x, x[1] = a4.y, x[2] = a4.z, x[3] = a4.w, x[4] = b4.x, x[5] = b4.y, x[6] = b4.z, x[7] = b4.w;
-        } else if (live && bulk) {
-#pragma unroll
-          for (int l = 0; l < 8; l++) x[l] = 8 * j + l < pr.d ? srow[8 * j + l] : 0.0f;
-        } else {
-#pragma unroll
-          for (int l = 0; l < 8; l++) x[l] = (live && 8 * j + l < pr.d) ? __ldg(xr + 8 * j + l) : 0.0f;
-        }
+      const float* stage = reinterpret_cast<const float*>(base + kTcOffS + (uint32_t)b * kTcS);
+      const int lpr = pr.d <= 32 ? 4 : 8;  // lanes per row
+      const int j = tid & (lpr - 1);
+      auto convert = [&](int row, const float (&x)[8]) {
         uint32_t hw[4], lw[4];
+        f32x2 s = 0;
 #pragma unroll
         for (int l = 0; l < 8; l += 2) {
           const __nv_bfloat162 h = __floats2bfloat162_rn(x[l], x[l + 1]);
           const float2 hf = __bfloat1622float2(h);
-          const __nv_bfloat162 lo = __floats2bfloat162_rn(x[l] - hf.x, x[l + 1] - hf.y);
+          const f32x2 xx = pack2(x[l], x[l + 1]);
+          float2 rest;
+          unpack2(fma2(pack2(hf.x, hf.y), kNegOne2, xx), rest.x, rest.y);  // x - hi
+          const __nv_bfloat162 lo = __floats2bfloat162_rn(rest.x, rest.y);
           hw[l / 2] = *reinterpret_cast<const uint32_t*>(&h);
           lw[l / 2] = *reinterpret_cast<const uint32_t*>(&lo);
-          pn[l] = fmaf(x[l], x[l], pn[l]);
-          pn[l + 1] = fmaf(x[l + 1], x[l + 1], pn[l + 1]);
+          s = fma2(xx, xx, s);
         }
-        const uint32_t off = (uint32_t)tid * 128u + ((uint32_t)(j ^ (tid & 7)) << 4);
+        const uint32_t off = (uint32_t)row * 128u + ((uint32_t)(j ^ (row & 7)) << 4);
         *reinterpret_cast<uint4*>(sAh + off) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
         *reinterpret_cast<uint4*>(sAl + off) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+        // the norm: two chains of 4 and a tree over the row's lanes (7 roundings on a
+        // path for d = 32, 8 above: within (ceil(d/8) + 3) u |x|^2)
+        float v, v1;
+        unpack2(s, v, v1);
+        v += v1;
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        if (lpr == 8) v += __shfl_xor_sync(0xffffffffu, v, 4);
+        if (j == 0) xn2s[slot * 128 + row] = v;
+      };
+      if (bulk && pr.d == 8 * lpr) {  // whole chunks of staged rows (past n: unread)
+        const float* src = stage + 8 * j;
+        for (int row = tid / lpr; row < kTcRows; row += 2 * (kTcLoaders / lpr)) {
+          float x[2][8];
+#pragma unroll
+          for (int u = 0; u < 2; u++) {
+            const float* s = src + (row + u * (kTcLoaders / lpr)) * pr.d;
+            const float4 a4 = *reinterpret_cast<const float4*>(s);
+            const float4 b4 = *reinterpret_cast<const float4*>(s + 4);
+            x[u][0] = a4.x, x[u][1] = a4.y, x[u][2] = a4.z, x[u][3] = a4.w;
+            x[u][4] = b4.x, x[u][5] = b4.y, x[u][6] = b4.z, x[u][7] = b4.w;
+          }
+#pragma unroll
+          for (int u = 0; u < 2; u++) convert(row + u * (kTcLoaders / lpr), x[u]);
+        }
+      } else {
+#pragma unroll 1
+        for (int row = tid / lpr; row < kTcRows; row += kTcLoaders / lpr) {
+          const bool live = pr.active && i0 + row < pr.n;
+          const float* xr = X + pr.x_off + (live ? i0 + row : 0) * pr.d;
+          float x[8];
+#pragma unroll
+          for (int l = 0; l < 8; l++) {
+            const int t = 8 * j + l;
+            x[l] = !live || t >= pr.d ? 0.0f : bulk ? stage[row * pr.d + t] : __ldg(xr + t);
+          }
+          convert(row, x);
+        }
       }
-      xn2s[b * 128 + tid] = ((pn[0] + pn[1]) + (pn[2] + pn[3])) + ((pn[4] + pn[5]) + (pn[6] + pn[7]));
       if (tid == 0) {
         ItemMeta m;
         m.n = pr.n;
@@ -675,33 +687,51 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
         m.L = pr.L;
         m.e_lo = pr.e_lo;
         m.cnt_off = pr.cnt_off;
-        meta[b] = m;
+        meta[slot] = m;
       }
       // generic-proxy smem writes -> visible to the tensor core's async proxy
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      tcx::mbar_arrive(&a_full[b]);
+      __syncwarp();
+      if (lane == 0) tcx::mbar_arrive(&a_full[b]);
     }
-    // a copy still in flight must not outlive the CTA: the last one armed on
-    // each staging buffer lands before the exit (also after an abort)
-    if (tid == 0) {
-      volatile int never = 0;
-      for (int s = 0; s < 2; s++)
-        if (issued[s] > 0 && !tcx::mbar_wait(&stage_full[s], (uint32_t)((issued[s] - 1) & 1), &never))
-          atomicOr(ta.status, DEV_TIMEOUT);
-    }
-  } else if (warp == 4) {
-    // ---- MMA issuer ---------------------------------------------------------
+  } else if (warp == 8) {
+    // ---- row copies and MMAs, one lane -----------------------------------------
     if (lane == 0) {
+      int issued[2] = {0, 0};  // copies (or plain arrivals) armed per staging buffer
+      BProb pr;
+      int64_t q_begin = 0, q_end = 0;
+      int q = -1;
+      // item lt's rows into staging buffer lt & 1
+      auto fetch = [&](int64_t lt) {
+        const int s = (int)(lt & 1);
+        issued[s]++;
+        if (it0 + lt >= q_end) {
+          q = problem_of(it0 + lt, q);
+          pr = probs[ta.tcp[q]];
+          q_begin = ta.item_begin[q];
+          q_end = ta.item_begin[q + 1];
+        }
+        const int64_t i0 = (it0 + lt - q_begin) * kTcRows;
+        const uint32_t by = bulk_bytes(pr, i0);
+        if (by) {
+          tcx::mbar_expect_tx(&stage_full[s], by);
+          tcx::bulk_load(base + kTcOffS + (uint32_t)s * kTcS, X + pr.x_off + i0 * pr.d, by, &stage_full[s]);
+        } else {
+          tcx::mbar_arrive(&stage_full[s]);
+        }
+      };
+      for (int64_t lt = 0; lt < 2 && lt < nlt; lt++) fetch(lt);
       for (int64_t lt = 0; lt < nlt && !*abort_flag; lt++) {
         const int b = (int)(lt & 1);
         const uint32_t ph = (uint32_t)((lt >> 1) & 1);
-        if (!tcx::mbar_wait(&a_full[b], ph, abort_flag)) {
+        if (!tcx::mbar_wait(&a_full[b], ph, abort_flag) ||
+            !tcx::mbar_wait(&item_done[b], ph ^ 1u, abort_flag)) {
           if (!*abort_flag) atomicOr(ta.status, DEV_TIMEOUT);
           *abort_flag = 1;
           break;
         }
         tcx::tc_fence_after();
-        const int kp = meta[b].kp;
+        const int kp = meta[lt & 3].kp;
         if (kp > 0) {
           unsigned char* sAh = base + (uint32_t)b * kTcA;
           const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kp >> 3) << 17) |
@@ -712,7 +742,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
           const uint64_t bl = tcx::smem_desc_sw128(tcx::smem_u32(sBl));
           const uint32_t d_tmem = tmem + (uint32_t)b * 256u;
           // K steps of 16 that hold data (the zero columns past d add nothing)
-          const int nks = (meta[b].d + 15) >> 4;
+          const int nks = (meta[lt & 3].d + 15) >> 4;
 #pragma unroll
           for (int kk = 0; kk < 4; kk++)
             if (kk < nks) tcx::umma_bf16(d_tmem, ah + 2 * kk, bh + 2 * kk, idesc, kk ? 1u : 0u);
@@ -724,19 +754,29 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
             if (kk < nks) tcx::umma_bf16(d_tmem, al + 2 * kk, bh + 2 * kk, idesc, 1u);
         }
         tcx::umma_commit(&acc_full[b]);
+        // the rows of this staging buffer have been converted (a_full)
+        if (lt + 2 < nlt) fetch(lt + 2);
       }
       // every MMA issued here has completed before TMEM is freed
       tcx::umma_commit(fin);
       volatile int never = 0;
       if (!tcx::mbar_wait(fin, 0, &never)) atomicOr(ta.status, DEV_TIMEOUT);
+      // a copy still in flight must not outlive the CTA: the last one armed on
+      // each staging buffer lands before the exit (also after an abort)
+      for (int s = 0; s < 2; s++)
+        if (issued[s] > 0 && !tcx::mbar_wait(&stage_full[s], (uint32_t)((issued[s] - 1) & 1), &never))
+          atomicOr(ta.status, DEV_TIMEOUT);
     }
   } else {
-    // ---- epilogue: warp w reads TMEM lanes 32 * (w % 4) .. +32 ---------------
+    // ---- epilogue: warp w reads TMEM lanes 32 * (w % 4) .. +32; warps 9-12 take the
+    // items of buffer 0, warps 13-16 those of buffer 1 -------------------------
     const int g = warp & 3;
     const int row = g * 32 + lane;
     const double u24 = 5.9604644775390625e-08;
-    for (int64_t lt = 0; lt < nlt; lt++) {
-      const int b = (int)(lt & 1);
+    const int b = (warp - 9) >> 2;
+    int last_d = -1;
+    float beta = 0.0f, gamma = 0.0f;  // error terms of a problem's d
+    for (int64_t lt = b; lt < nlt; lt += 2) {
       const uint32_t ph = (uint32_t)((lt >> 1) & 1);
       bool ok = !*abort_flag && tcx::mbar_wait(&acc_full[b], ph, abort_flag);
       if (!ok) {
@@ -745,16 +785,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
       }
       if (!__all_sync(0xffffffffu, ok)) break;  // warp-uniform exit
       tcx::tc_fence_after();
-      const ItemMeta mt = meta[b];
+      const int slot = (int)(lt & 3);
+      const ItemMeta mt = meta[slot];
       const int kp = mt.kp;
       const int64_t i = (int64_t)mt.i0 + row;
       const bool live = kp > 0 && i < mt.n;
       // the row's current label, fetched while the screen runs
       const int old = live ? (first ? -1 : labels[mt.lab_off + i]) : -1;
-      const float cmax0 = cmaxs[0];
-      const float nx = xn2s[b * 128 + row];
-      const float beta = (float)(((mt.d + 7) / 8 + 3 + 9) * u24 * 1.01);
-      const float gamma = (float)((mt.d + 4) * u24 * 1.01);
+      const float cmax0 = cmaxs[0], cmax1 = cmaxs[1];
+      const float nx = xn2s[slot * 128 + row];
+      if (mt.d != last_d) {
+        last_d = mt.d;
+        beta = (float)(((mt.d + 7) / 8 + 3 + 9) * u24 * 1.01);
+        gamma = (float)((mt.d + 4) * u24 * 1.01);
+      }
       const uint32_t taddr = tmem + ((uint32_t)(g * 32) << 16) + (uint32_t)b * 256u;
       const float xl = sqrtf(nx);
       float best = __int_as_float(0x7f800000);
@@ -765,77 +809,119 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
       uint32_t cmask[8];
       uint32_t cm_set = 0;
       if (kp > 0) {
-        // screen, two passes over the TMEM columns (32 per wait).  Pass 1: the
-        // smallest screen value (four independent running minima over the
-        // columns of each residue mod 4; the padding columns past k read +inf
-        // norms).  The best centre's upper bound is taken with the problem's
-        // norm maxima (at least its own error term), so it needs no column
-        // index.  Pass 2: the first column holding the smallest value is the
-        // best centre (first index wins ties, as in a scan), and every other
-        // column whose lower bound reaches the bound is a candidate; columns
-        // above T cannot reach it with the largest error of the problem.
-        float b4[4] = {best, best, best, best};
-        for (int c0 = 0; c0 < kp; c0 += 32) {
-          uint32_t r[2][16];
+        // Screen over the TMEM columns, 32 per wait, without branches on a column's
+        // value.  Pass 1: the smallest screen value (padding columns past k read
+        // +inf norms).  The best centre's upper bound hi_b takes the problem's norm
+        // maxima (at least its own error term), so it needs no column index, and no
+        // column above T reaches it with the largest error of the problem.  Pass 2:
+        // the columns up to T.  A row with one such column is decided.  Pass 3, for
+        // warps with another row: the first column holding the smallest value is the
+        // best centre (first index wins ties, as in a scan), and every other column
+        // whose own lower bound reaches the bound is a candidate.
+        const f32x2 nx2 = pack2(nx, nx), m2 = pack2(-2.0f, -2.0f);
+        uint32_t r[2][16];
+        auto columns = [&](int c0) {
 #pragma unroll
           for (int h = 0; h < 2; h++)
             if (c0 + 16 * h < kp) tcx::tmem_ld16_nowait(taddr + c0 + 16 * h, r[h]);
           tcx::tmem_ld_wait();
 #pragma unroll
           for (int h = 0; h < 2; h++) tcx::tmem_regs_ready(r[h]);
+        };
+        // screen values fma(-2, dot, |x|^2 + |c|^2) of columns c0 + 16 h + 4 v ..
+        auto screen4 = [&](int c, const uint32_t* q, float (&dt)[4], float (&cc)[4]) {
+          const float4 c4 = *reinterpret_cast<const float4*>(cn2s + c);
+          cc[0] = c4.x, cc[1] = c4.y, cc[2] = c4.z, cc[3] = c4.w;
+#pragma unroll
+          for (int u = 0; u < 4; u += 2)
+            unpack2(fma2(m2, pack2(__uint_as_float(q[u]), __uint_as_float(q[u + 1])),
+                         add2(nx2, pack2(cc[u], cc[u + 1]))),
+                    dt[u], dt[u + 1]);
+        };
+        float b4[4] = {best, best, best, best};
+        for (int c0 = 0; c0 < kp; c0 += 32) {
+          columns(c0);
 #pragma unroll
           for (int h = 0; h < 2; h++) {
             if (c0 + 16 * h >= kp) break;
 #pragma unroll
             for (int v = 0; v < 4; v++) {
-              const float4 c4 = *reinterpret_cast<const float4*>(cn2s + c0 + 16 * h + 4 * v);
-              const float cc[4] = {c4.x, c4.y, c4.z, c4.w};
+              float dt[4], cc[4];
+              screen4(c0 + 16 * h + 4 * v, r[h] + 4 * v, dt, cc);
 #pragma unroll
-              for (int u = 0; u < 4; u++)
-                b4[u] = fminf(b4[u], fmaf(-2.0f, __uint_as_float(r[h][4 * v + u]), nx + cc[u]));
+              for (int u = 0; u < 4; u++) b4[u] = fminf(b4[u], dt[u]);
             }
           }
         }
         best = fminf(fminf(b4[0], b4[1]), fminf(b4[2], b4[3]));
-        const float amax = (ta.alpha * xl * sqrtf(cmax0) + beta * (nx + cmax0)) * (1.0f + gamma);
+        const float amax = (ta.alpha * xl * cmax1 + beta * (nx + cmax0)) * (1.0f + gamma);
         const float hi_b = best + amax + gamma * fabsf(best);
-        const float T = (hi_b + amax) * (1.0f + 2.0f * gamma) * (1.0f + 9.5367431640625e-07f);
-        bool found = false;
+        const float T0 = (hi_b + amax) * (1.0f + 2.0f * gamma) * (1.0f + 9.5367431640625e-07f);
+        const float T = T0 > 0.0f ? T0 : __int_as_float(0x7f800000);
+        // One instruction per column: the sign of dt - T', T' the next value above T,
+        // shifted into a word.  Finite T: every norm, screen value and bound of the
+        // row is finite (T covers the largest of each).
+        const bool finite = T < __int_as_float(0x7f800000);
+        const float nt = -__int_as_float(__float_as_int(T) + (finite ? 1 : 0));
+        const f32x2 nt2 = pack2(nt, nt);
+        int near = 0;  // columns up to T
         for (int c0 = 0; c0 < kp; c0 += 32) {
-          uint32_t bits = 0;
-          uint32_t r[2][16];
-#pragma unroll
-          for (int h = 0; h < 2; h++)
-            if (c0 + 16 * h < kp) tcx::tmem_ld16_nowait(taddr + c0 + 16 * h, r[h]);
-          tcx::tmem_ld_wait();
-#pragma unroll
-          for (int h = 0; h < 2; h++) tcx::tmem_regs_ready(r[h]);
+          uint32_t bits = 0;  // the last column at bit 0
+          columns(c0);
 #pragma unroll
           for (int h = 0; h < 2; h++) {
             if (c0 + 16 * h >= kp) break;
 #pragma unroll
             for (int v = 0; v < 4; v++) {
-              const float4 c4 = *reinterpret_cast<const float4*>(cn2s + c0 + 16 * h + 4 * v);
-              const float cc[4] = {c4.x, c4.y, c4.z, c4.w};
+              float dt[4], cc[4];
+              screen4(c0 + 16 * h + 4 * v, r[h] + 4 * v, dt, cc);
 #pragma unroll
-              for (int u = 0; u < 4; u++) {
-                const int col = c0 + 16 * h + 4 * v + u;
-                const float dt = fmaf(-2.0f, __uint_as_float(r[h][4 * v + u]), nx + cc[u]);
-                if (!found && dt == best) {
-                  found = true;
-                  bj = col;
-                } else if (!(T > 0.0f) || !(dt > T)) {  // padding columns (+inf) only when T <= 0
-                  const float e =
-                      (ta.alpha * xl * cns[col] + beta * (nx + cc[u])) * (1.0f + gamma) + gamma * fabsf(dt);
-                  if (!(dt - e > hi_b)) bits |= 1u << (16 * h + 4 * v + u);
-                }
+              for (int u = 0; u < 4; u += 2) {
+                float e0, e1;
+                unpack2(add2(pack2(dt[u], dt[u + 1]), nt2), e0, e1);
+                bits = __funnelshift_l(__float_as_uint(e0), bits, 1);
+                bits = __funnelshift_l(__float_as_uint(e1), bits, 1);
               }
             }
           }
-          if (bits) {
-            undecided = true;
-            cmask[c0 >> 5] = bits;
-            cm_set |= 1u << (c0 >> 5);
+          near += __popc(bits);
+          if (bits) bj = min(c0 + 32, kp) - __ffs(bits);
+        }
+        bool found = finite && near == 1;
+        if (__any_sync(0xffffffffu, live && !found)) {
+          bj = 0;
+          found = false;
+          for (int c0 = 0; c0 < kp; c0 += 32) {
+            uint32_t bits = 0, eq = 0;
+            columns(c0);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              if (c0 + 16 * h >= kp) break;
+#pragma unroll
+              for (int v = 0; v < 4; v++) {
+                float dt[4], cc[4];
+                screen4(c0 + 16 * h + 4 * v, r[h] + 4 * v, dt, cc);
+                const float4 s4 = *reinterpret_cast<const float4*>(cns + c0 + 16 * h + 4 * v);
+                const float ss[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                  const float e = (ta.alpha * xl * ss[u] + beta * (nx + cc[u])) * (1.0f + gamma) + gamma * fabsf(dt[u]);
+                  const uint32_t bit = 1u << (16 * h + 4 * v + u);
+                  eq |= dt[u] == best ? bit : 0u;
+                  bits |= !(dt[u] > T) && !(dt[u] - e > hi_b) ? bit : 0u;
+                }
+              }
+            }
+            if (!found && eq) {
+              found = true;
+              bj = c0 + __ffs(eq) - 1;
+              bits &= ~(eq & (0u - eq));
+            }
+            if (bits) {
+              undecided = true;
+              cmask[c0 >> 5] = bits;
+              cm_set |= 1u << (c0 >> 5);
+            }
           }
         }
         // no column equal to the minimum (a NaN screen value): the re-score
@@ -848,30 +934,38 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
       }
       // the item's accumulator, tile and parameters are no longer read
       tcx::tc_fence_before();
-      tcx::mbar_arrive(&item_done[b]);
+      __syncwarp();
+      if (lane == 0) tcx::mbar_arrive(&item_done[b]);
       if (kp == 0) continue;
       const int p = mt.p;
       const int lab = bj;
-      {
-        const unsigned um = __ballot_sync(0xffffffffu, live && undecided);
-        if (lane == 0 && um) atomicAdd(ta.undecided, (unsigned long long)__popc(um));
+      const bool chg = live && !undecided && lab != old;
+      const unsigned um = __ballot_sync(0xffffffffu, live && undecided);
+      const unsigned cm = __ballot_sync(0xffffffffu, chg);
+      // places on the undecided and the change list, both asked for before either
+      // answer is used
+      int u_at = 0, c_at = 0;
+      if (lane == 0) {
+        if (um) u_at = atomicAdd(ta.und_n, __popc(um));
+        if (!first && cm) c_at = atomicAdd(ta.chg_n, __popc(cm));
+        if (um) atomicAdd(ta.undecided, (unsigned long long)__popc(um));
+        if (!first && cm) atomicAdd(&pchg[p], __popc(cm));
       }
+      const unsigned below = (1u << lane) - 1u;
+      u_at = __shfl_sync(0xffffffffu, u_at, 0) + __popc(um & below);
+      c_at = __shfl_sync(0xffffffffu, c_at, 0) + __popc(cm & below);
       if (live && undecided) {
         // the exact re-score kernel decides this row among its candidates
         // and the screen's best
-        const int u = atomicAdd(ta.und_n, 1);
-        ta.und_p[u] = p;
-        ta.und_i[u] = (int32_t)i;
-        uint32_t* um = ta.und_m + (int64_t)u * ta.und_w;
+        ta.und_p[u_at] = p;
+        ta.und_i[u_at] = (int32_t)i;
+        uint32_t* words = ta.und_m + (int64_t)u_at * ta.und_w;
         for (int w = 0; w < ta.und_w; w++) {
           uint32_t m = ((cm_set >> w) & 1u) ? cmask[w] : 0u;
           if (w == (bj >> 5)) m |= 1u << (bj & 31);
-          um[w] = m;
+          words[w] = m;
         }
       }
-      const bool chg = live && !undecided && lab != old;
-      const unsigned cm = __ballot_sync(0xffffffffu, chg);
-      if (!first && lane == 0 && cm) atomicAdd(&pchg[p], __popc(cm));
       if (chg) {
         labels[mt.lab_off + i] = lab;
         atomicAdd(&counts[mt.cnt_off + lab], 1);
@@ -882,22 +976,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
       if (first) continue;
       // later passes: the changed rows go to the change list (bucketed and
       // summed after the pass) while it has room
-      bool listed = false;
-      {
-        const unsigned cmw = __ballot_sync(0xffffffffu, chg);
-        if (cmw) {
-          int at = 0;
-          if (lane == 0) at = atomicAdd(ta.chg_n, __popc(cmw));
-          at = __shfl_sync(0xffffffffu, at, 0) + __popc(cmw & ((1u << lane) - 1u));
-          if (chg && at < ta.chg_cap) {
-            listed = true;
-            ta.chg_row[at] = (int32_t)i;
-            ta.chg_new[at] = mt.cnt_off + lab;
-            ta.chg_old[at] = mt.cnt_off + old;
-            atomicAdd(&ta.hist[2 * (mt.cnt_off + lab)], 1);
-            atomicAdd(&ta.hist[2 * (mt.cnt_off + old) + 1], 1);
-          }
-        }
+      const bool listed = chg && c_at < ta.chg_cap;
+      if (listed) {
+        ta.chg_row[c_at] = (int32_t)i;
+        ta.chg_new[c_at] = mt.cnt_off + lab;
+        ta.chg_old[c_at] = mt.cnt_off + old;
+        atomicAdd(&ta.hist[2 * (mt.cnt_off + lab)], 1);
+        atomicAdd(&ta.hist[2 * (mt.cnt_off + old) + 1], 1);
       }
       // the others' coordinates into the exact sums: the warp takes the
       // rows that enter one cluster (or leave one) together -- lanes over
@@ -943,7 +1028,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) batched_tc_assign_kernel(
   }
   tcx::tc_fence_before();
   __syncthreads();
-  if (warp == 4) {
+  if (warp == 8) {
     tcx::tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
@@ -1599,14 +1684,14 @@ extern "C" int fuelg_kmeans_batched(fuelg_kmeans_problem* probs, int32_t count, 
   }
   auto grid_for = [&](int b) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(items, (int64_t)sms * b)); };
   // one persistent screen CTA per SM, each over a contiguous range of items of
-  // equal estimated cost (row loads + an epilogue that grows with the centres)
+  // equal estimated cost (cycles per item by k: 3200 at 30, 3700 at 48, 4700 at 113)
   const unsigned tc_grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(tc_items, (int64_t)sms));
   {
     std::vector<double> icost(ntc);
     double total = 0.0;
     for (int q = 0; q < ntc; q++) {
       const int kp = (hp[tcp[q]].k + 15) & ~15;
-      icost[q] = 64.0 + 2.0 * kp;
+      icost[q] = 200.0 + 2.0 * kp;
       total += icost[q] * (tc_begin[q + 1] - tc_begin[q]);
     }
     std::vector<int64_t> cb(tc_grid + 1, 0);
