@@ -125,12 +125,52 @@ __device__ __forceinline__ void add_coord(unsigned long long* __restrict__ dst, 
   }
 }
 
+// The squared distances from x (each coordinate twice) to two centres c (their
+// coordinates interleaved), two lanes of one packed chain: the operation
+// sequence of exact_dist_fn<KIND, ORDER, D> for D = 2 or 8.  nz is kNegZero2, as
+// an argument: a product plus an explicit -0 stays a product of its own.
+template <int KIND, int ORDER, int D>
+__device__ __forceinline__ f32x2 exact_dist_pair(const f32x2 (&x)[D], const f32x2* __restrict__ c, f32x2 nz) {
+  static_assert(D == 2 || D == 8, "");
+  static_assert(KIND == KIND_SQDIST || KIND == KIND_PAIRWISE, "");
+  constexpr bool fma_chain = KIND == KIND_PAIRWISE && ORDER == ORDER_X86 && D >= 4;
+  constexpr bool tree = KIND == KIND_SQDIST && ORDER == ORDER_X86 && D == 8;
+  f32x2 sq[D];
+  f32x2 s = 0;
+#pragma unroll
+  for (int t = 0; t < D; t += 2) {
+    const ulonglong2 cc = *reinterpret_cast<const ulonglong2*>(c + t);
+    const f32x2 d0 = fma2(cc.x, kNegOne2, x[t]), d1 = fma2(cc.y, kNegOne2, x[t + 1]);
+    if (fma_chain) {
+      s = t == 0 ? fma2(d0, d0, nz) : fma2(d0, d0, s);
+      s = fma2(d1, d1, s);
+    } else {
+      sq[t] = fma2(d0, d0, nz);
+      sq[t + 1] = fma2(d1, d1, nz);
+    }
+  }
+  if constexpr (tree) {
+    return add2(add2(add2(sq[0], sq[4]), add2(sq[1], sq[5])), add2(add2(sq[2], sq[6]), add2(sq[3], sq[7])));
+  } else if constexpr (!fma_chain) {
+    s = sq[0];  // (+0 + a square is the square)
+#pragma unroll
+    for (int t = 1; t < D; t++) s = add2(s, sq[t]);
+  }
+  return s;
+}
+
 // One iteration over all problems: assignment + sum updates of changed points.
-template <int KIND, int ORDER>
+// Problems of 2 or 8 dimensions whose centres fit (every such problem up to 2048
+// centres): two centres per packed step, their coordinates interleaved in shared
+// memory.  WIDE: some problem has 32 or 64 dimensions, whose rows are held in
+// registers (128 per thread; 64 without).  Bound by FP32 issue and, in the first
+// passes, by the adds of changed rows: a later pass over 10.3 million rows of 2 or
+// 8 dimensions, k to 256: 0.90 -> 0.56 ms against one centre at a time.
+template <int KIND, int ORDER, bool WIDE>
 __global__ void __launch_bounds__(kItemRows) batched_assign_kernel(
     const BProb* __restrict__ probs, int P, int items_total, const float* __restrict__ X,
     const float* __restrict__ C, int32_t* __restrict__ labels, unsigned long long* __restrict__ limbs,
-    int32_t* __restrict__ counts, int32_t* __restrict__ pchg, int first, int64_t work_total, int ccap) {
+    int32_t* __restrict__ counts, int32_t* __restrict__ pchg, int first, int64_t work_total, int ccap, f32x2 nz) {
   extern __shared__ __align__(16) unsigned char smem_b[];
   float* cs = reinterpret_cast<float*>(smem_b);                                           // [ccap]
   unsigned long long* agg = reinterpret_cast<unsigned long long*>(cs + ccap);            // [kAggCap]
@@ -143,7 +183,7 @@ __global__ void __launch_bounds__(kItemRows) batched_assign_kernel(
                                                  (int64_t)((__int128)work_total * (blockIdx.x + 1) / gridDim.x));
   int p = -1;
   BProb pr{};
-  bool staged = false, use_agg = false;
+  bool staged = false, paired = false, use_agg = false;
   // flush this CTA's partial sums / counts / change count of problem p
   auto flush = [&]() {
     __syncthreads();
@@ -169,11 +209,20 @@ __global__ void __launch_bounds__(kItemRows) batched_assign_kernel(
       __syncthreads();
       p = lo;
       pr = probs[p];
-      staged = pr.k * pr.d <= ccap;
+      staged = ((pr.k + 1) & ~1) * pr.d <= ccap;
+      paired = staged && (pr.d == 2 || pr.d == 8);
       use_agg = pr.k * pr.d * pr.L <= kAggCap && pr.k <= 256;
       if (pr.active) {
-        if (staged)
+        if (paired) {
+          // centres 2 j and 2 j + 1 interleaved; an odd last one with a NaN, which is
+          // never nearer
+          for (int e = threadIdx.x; e < ((pr.k + 1) & ~1) * pr.d; e += blockDim.x) {
+            const int c = e / pr.d, t = e - c * pr.d;
+            cs[((c >> 1) * pr.d + t) * 2 + (c & 1)] = c < pr.k ? C[pr.c_off + e] : __int_as_float(0x7fffffff);
+          }
+        } else if (staged) {
           for (int e = threadIdx.x; e < pr.k * pr.d; e += blockDim.x) cs[e] = C[pr.c_off + e];
+        }
         if (use_agg) {
           for (int e = threadIdx.x; e < pr.k * pr.d * pr.L; e += blockDim.x) agg[e] = 0;
           for (int e = threadIdx.x; e < pr.k; e += blockDim.x) aggc[e] = 0;
@@ -216,12 +265,37 @@ __global__ void __launch_bounds__(kItemRows) batched_assign_kernel(
           }
         }
       };
-      switch (pr.d) {
-        case 2: scan(Dim<2>{}); break;
-        case 8: scan(Dim<8>{}); break;
-        case 32: scan(Dim<32>{}); break;
-        case 64: scan(Dim<64>{}); break;
-        default:
+      auto scan_pairs = [&](auto dimc) {
+        constexpr int DD = decltype(dimc)::value;
+        f32x2 x[DD];
+#pragma unroll
+        for (int t = 0; t < DD; t++) {
+          const float v = __ldg(xr + t);
+          x[t] = pack2(v, v);
+        }
+        const f32x2* cp = reinterpret_cast<const f32x2*>(cs);
+        float d0, d1;
+        unpack2(exact_dist_pair<KIND, ORDER, DD>(x, cp, nz), d0, d1);
+        bd = d0;  // the first centre, whatever its distance
+        best = 0;
+#pragma unroll 2
+        for (int c = 0; c < pr.k; c += 2, cp += DD) {
+          unpack2(exact_dist_pair<KIND, ORDER, DD>(x, cp, nz), d0, d1);
+          if (d0 < bd) {
+            bd = d0;
+            best = c;
+          }
+          if (d1 < bd) {
+            bd = d1;
+            best = c + 1;
+          }
+        }
+      };
+      if (paired && pr.d == 2) scan_pairs(Dim<2>{});
+      else if (paired) scan_pairs(Dim<8>{});
+      else if (WIDE && pr.d == 32) scan(Dim<32>{});
+      else if (WIDE && pr.d == 64) scan(Dim<64>{});
+      else {
           for (int c = 0; c < pr.k; c++) {
             const float dv = exact_dist_scalar<KIND, ORDER>(xr, C + pr.c_off + (int64_t)c * pr.d, pr.d);
             if (best < 0 || dv < bd) {
@@ -1578,7 +1652,7 @@ extern "C" int fuelg_kmeans_batched(fuelg_kmeans_problem* probs, int32_t count, 
   // the tensor-core screen): more resident CTAs when their centres are small
   int ccap = 4;
   for (int p = 0; p < P; p++)
-    if (!hp[p].tc) ccap = std::max<int64_t>(ccap, std::min<int64_t>(kCentreCap, (int64_t)hp[p].k * hp[p].d));
+    if (!hp[p].tc) ccap = std::max<int64_t>(ccap, std::min<int64_t>(kCentreCap, (int64_t)((hp[p].k + 1) & ~1) * hp[p].d));
   ccap = (ccap + 3) & ~3;
   // With tensor-core problems in the batch the CUDA-core kernel runs beside the
   // screen (its own stream, joined before the centre update): with the centres
@@ -1587,10 +1661,15 @@ extern "C" int fuelg_kmeans_batched(fuelg_kmeans_problem* probs, int32_t count, 
   // epilogue leaves.
   const bool concurrent = items > 0 && tc_items > 0;
   const size_t smem = sizeof(float) * ccap + sizeof(unsigned long long) * kAggCap + sizeof(int) * 256;
-  auto k_init = order == FUELG_ORDER_X86 ? batched_assign_kernel<KIND_PAIRWISE, ORDER_X86>
-                                         : batched_assign_kernel<KIND_PAIRWISE, ORDER_ARM>;
-  auto k_iter = order == FUELG_ORDER_X86 ? batched_assign_kernel<KIND_SQDIST, ORDER_X86>
-                                         : batched_assign_kernel<KIND_SQDIST, ORDER_ARM>;
+  bool wide = false;
+  for (int p = 0; p < P; p++) wide = wide || (!hp[p].tc && (hp[p].d == 32 || hp[p].d == 64));
+  auto assign = [&](auto kind, bool x86) {
+    constexpr int K = decltype(kind)::value;
+    return x86 ? (wide ? batched_assign_kernel<K, ORDER_X86, true> : batched_assign_kernel<K, ORDER_X86, false>)
+               : (wide ? batched_assign_kernel<K, ORDER_ARM, true> : batched_assign_kernel<K, ORDER_ARM, false>);
+  };
+  auto k_init = assign(Dim<KIND_PAIRWISE>{}, order == FUELG_ORDER_X86);
+  auto k_iter = assign(Dim<KIND_SQDIST>{}, order == FUELG_ORDER_X86);
   FUELG_CUDA(cudaFuncSetAttribute(k_init, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   FUELG_CUDA(cudaFuncSetAttribute(k_iter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   auto t_init = order == FUELG_ORDER_X86 ? batched_tc_assign_kernel<KIND_PAIRWISE, ORDER_X86>
@@ -1727,11 +1806,11 @@ extern "C" int fuelg_kmeans_batched(fuelg_kmeans_problem* probs, int32_t count, 
       if (first)
         k_init<<<grid, kItemRows, smem, sc>>>(dProbs.as<BProb>(), P, (int)items, dX.as<float>(), dC.as<float>(),
                                              dLab.as<int32_t>(), dLimbs.as<unsigned long long>(), dCnt.as<int32_t>(),
-                                             dPchg.as<int32_t>(), 1, work, ccap);
+                                             dPchg.as<int32_t>(), 1, work, ccap, kNegZero2);
       else
         k_iter<<<grid, kItemRows, smem, sc>>>(dProbs.as<BProb>(), P, (int)items, dX.as<float>(), dC.as<float>(),
                                              dLab.as<int32_t>(), dLimbs.as<unsigned long long>(), dCnt.as<int32_t>(),
-                                             dPchg.as<int32_t>(), 0, work, ccap);
+                                             dPchg.as<int32_t>(), 0, work, ccap, kNegZero2);
       note_launch();
     }
     if (tc_items > 0) {
