@@ -38,6 +38,7 @@
 #include "fuelg_prep.cuh"
 #include "fuelg_sums.cuh"
 #include "fuelg_tc_common.cuh"
+#include "fuelg_tile.cuh"
 
 namespace fuelg {
 
@@ -288,12 +289,17 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       sncd[j] = j < a.k ? nc2 : __int_as_float(0x7f800000);
     }
     named_bar_sync(1, BM);
-    for (int j = 0; j < a.k; j++) {
+    // (NaN norms are not finite; a maximum that missed one is then unused)
+    for (int j = lane; j < a.k; j += 32) {
       const float s2 = snc[j], c1 = scn[j];
       cta_finite = cta_finite && s2 < 0x1p124f && c1 < 0x1p62f;
       sncmax = fmaxf(sncmax, s2);
       scnmax = fmaxf(scnmax, c1);
     }
+    cta_finite = __all_sync(0xffffffffu, cta_finite);
+    // (non-negative: ordered like their bit patterns)
+    sncmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(sncmax)));
+    scnmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(scnmax)));
   }
 
   if (warp == 0) {
@@ -448,222 +454,168 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       tc_fence_after();
       const uint32_t acc_cols = (BLO && a.sep_lo ? 2u : 1u) * (uint32_t)a.kp;
       const uint32_t taddr = tmem_base + ((uint32_t)(g * 32) << 16) + buf * acc_cols;
-      float best = __int_as_float(0x7f800000), best_dot = 0.0f;
+      // Screen over the TMEM columns, 32 per wait, without branches on a column's
+      // value: dt_c = fma(-2, v_c, |x|^2 + |c|^2), +inf for padding columns.
+      // (Scans with a branch per column above 64 centres: 20 passes over 100 000 x 64,
+      // k = 200 3.83 -> 1.76 ms, 200 000 x 32, k = 128 4.56 -> 1.99, 76 000 x 784, k =
+      // 250 4.33 -> 2.92; up to 64 centres equal to the tournament tree this replaced,
+      // which the row loads and the update kernels bound.  With the best centre's own
+      // bound in pass 3, one sweep more, 1 to 4 % slower for 6 to 11 % fewer re-scores.)
+      float best = __int_as_float(0x7f800000);
       int bj = 0;
       uint64_t m0 = 0, m1 = 0, m2 = 0, m3 = 0;
-      if (a.kp <= 64) {
-        // Pass 1 without branches, per 32 columns (TMEM -> registers): the
-        // screen values dt_c = fma(-2, v_c, nxi + snc_c) (padding columns: +inf
-        // through sncd) reduced by a tree that keeps the smallest value, its
-        // first index and dot product, and the second smallest value (the left
-        // operand wins ties, so the first index wins, as in a scan).
-        float second = __int_as_float(0x7f800000), vmax = 0.0f;
+      const f32x2 nx2 = pack2(nxi, nxi), mtwo = pack2(-2.0f, -2.0f);
+      uint32_t rh[2][16], rl[2][16];
+      auto columns = [&](int c0) {
 #pragma unroll
-        for (int r = 0; r < 2; r++) {
-          if (32 * r >= a.kp) break;
-          uint32_t rh[2][16], rl[2][16];
+        for (int h = 0; h < 2; h++)
+          if (c0 + 16 * h < a.kp) {
+            tmem_ld16_nowait(taddr + c0 + 16 * h, rh[h]);
+            if (BLO && a.sep_lo) tmem_ld16_nowait(taddr + a.kp + c0 + 16 * h, rl[h]);
+          }
+        tmem_ld_wait();
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          tmem_regs_ready(rh[h]);
+          if (BLO && a.sep_lo) tmem_regs_ready(rl[h]);
+        }
+        // the dot products, in rh
+        if (BLO && a.sep_lo) {
 #pragma unroll
           for (int h = 0; h < 2; h++)
-            if (32 * r + 16 * h < a.kp) {
-              tmem_ld16_nowait(taddr + 32 * r + 16 * h, rh[h]);
-              if (BLO && a.sep_lo) tmem_ld16_nowait(taddr + a.kp + 32 * r + 16 * h, rl[h]);
+#pragma unroll
+            for (int u = 0; u < 16; u += 2) {
+              float v0, v1;
+              unpack2(add2(pack2(__uint_as_float(rh[h][u]), __uint_as_float(rh[h][u + 1])),
+                           pack2(__uint_as_float(rl[h][u]), __uint_as_float(rl[h][u + 1]))),
+                      v0, v1);
+              rh[h][u] = __float_as_uint(v0);
+              rh[h][u + 1] = __float_as_uint(v1);
             }
-          tmem_ld_wait();
+        }
+      };
+      // dt of columns c0 + 16 h + 4 q ..
+      auto screen4 = [&](int c0, int h, int q, float (&dt)[4], float (&cc)[4]) {
+        const float4 c4 = *reinterpret_cast<const float4*>(sncd + c0 + 16 * h + 4 * q);
+        cc[0] = c4.x, cc[1] = c4.y, cc[2] = c4.z, cc[3] = c4.w;
 #pragma unroll
-          for (int h = 0; h < 2; h++) {
-            tmem_regs_ready(rh[h]);
-            if (BLO && a.sep_lo) tmem_regs_ready(rl[h]);
-          }
-          float v[32], m[32], dv[32], s2[16];
-          int id[32];
+        for (int u = 0; u < 4; u += 2)
+          unpack2(fma2(mtwo, pack2(__uint_as_float(rh[h][4 * q + u]), __uint_as_float(rh[h][4 * q + u + 1])),
+                       add2(nx2, pack2(cc[u], cc[u + 1]))),
+                  dt[u], dt[u + 1]);
+      };
+      // Pass 1: the smallest value, and the largest dot product (nonnegative data)
+      float b4[4] = {best, best, best, best};
+      float vmax = 0.0f;
+      for (int c0 = 0; c0 < a.kp; c0 += 32) {
+        columns(c0);
 #pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const bool ld = 32 * r + 16 * h < a.kp;
+        for (int h = 0; h < 2; h++) {
+          if (c0 + 16 * h >= a.kp) break;
 #pragma unroll
-            for (int j = 0; j < 16; j++) {
-              float x = ld ? __uint_as_float(rh[h][j]) : 0.0f;
-              if (BLO && a.sep_lo && ld) x += __uint_as_float(rl[h][j]);
-              v[16 * h + j] = x;
-            }
-          }
-          const float4* sd4 = reinterpret_cast<const float4*>(sncd + 32 * r);
+          for (int q = 0; q < 4; q++) {
+            float dt[4], cc[4];
+            screen4(c0, h, q, dt, cc);
 #pragma unroll
-          for (int q = 0; q < 8; q++) {
-            const float4 s4 = sd4[q];
-            m[4 * q + 0] = fmaf(-2.0f, v[4 * q + 0], nxi + s4.x);
-            m[4 * q + 1] = fmaf(-2.0f, v[4 * q + 1], nxi + s4.y);
-            m[4 * q + 2] = fmaf(-2.0f, v[4 * q + 2], nxi + s4.z);
-            m[4 * q + 3] = fmaf(-2.0f, v[4 * q + 3], nxi + s4.w);
-          }
-#pragma unroll
-          for (int c = 0; c < 32; c++) {
-            dv[c] = v[c];
-            id[c] = 32 * r + c;
-          }
-#pragma unroll
-          for (int c = 0; c < 32; c += 2) {
-            const bool rt = m[c + 1] < m[c];
-            s2[c >> 1] = rt ? m[c] : m[c + 1];
-            m[c] = rt ? m[c + 1] : m[c];
-            id[c] = rt ? id[c + 1] : id[c];
-            dv[c] = rt ? dv[c + 1] : dv[c];
-          }
-#pragma unroll
-          for (int w = 2; w < 32; w <<= 1)
-#pragma unroll
-            for (int c = 0; c < 32; c += 2 * w) {
-              const bool rt = m[c + w] < m[c];
-              const float lose = rt ? m[c] : m[c + w];
-              s2[c >> 1] = min3_f32(lose, s2[c >> 1], s2[(c + w) >> 1]);
-              m[c] = rt ? m[c + w] : m[c];
-              id[c] = rt ? id[c + w] : id[c];
-              dv[c] = rt ? dv[c + w] : dv[c];
-            }
-          if (r == 0) {
-            best = m[0];
-            bj = id[0];
-            best_dot = dv[0];
-            second = s2[0];
-          } else {
-            const bool rt = m[0] < best;
-            second = min3_f32(rt ? best : m[0], second, s2[0]);
-            best = rt ? m[0] : best;
-            bj = rt ? id[0] : bj;
-            best_dot = rt ? dv[0] : best_dot;
+            for (int u = 0; u < 4; u++) b4[u] = fminf(b4[u], dt[u]);
           }
           if (nonneg) {
-            float mx = vmax;
 #pragma unroll
-            for (int c = 0; c < 32; c += 2) mx = max3_f32(mx, v[c], v[c + 1]);
-            vmax = mx;
-          }
-        }
-        const float sb = nonneg ? fmaxf(best_dot, 0.0f) * a.s_scale : xni * scn[bj];
-        const float eb = (a.alpha * sb + a.beta * (nxi + snc[bj])) * (1.0f + a.gamma) + a.gamma * fabsf(best);
-        const float hi = best + eb;
-        // Every other column j has dt_j >= second, and its rounded bound e_j
-        // (at most five roundings of non-negative terms) stays below
-        // (C + gamma |dt_j|)(1 + 2^-24)^5, C = the bound's other terms at the
-        // largest S_j and snc_j; t - gamma' |t| grows with t, so with
-        // tb >= (C + gamma |second|)(1 + 2^-18) a value second - tb two ulps
-        // above hi makes the per-column test below pass for every j.  Finite
-        // norms below 2^124 keep every dt finite.
-        constexpr float kInfl = 1.0f + 0x1p-18f;
-        const float smax = nonneg ? fmaxf(vmax, 0.0f) * a.s_scale : xni * scnmax;
-        const float cmax = (a.alpha * smax + a.beta * (nxi + sncmax)) * (1.0f + a.gamma) * kInfl;
-        const float tb = fmaf(a.gamma * kInfl, fabsf(second), cmax);
-        const float hu = __fadd_ru(__fmaf_ru(fabsf(hi), 0x1p-22f, hi), 0x1p-125f);
-        const bool easy = cta_finite && nxi < 0x1p124f && (second - tb) >= hu;
-        if (__any_sync(0xffffffffu, !easy)) {
-          // pass 2: every other centre whose lower bound reaches the best's
-          // upper bound (the columns re-read from TMEM, 32 per wait)
-          uint32_t blo = 0, bhi = 0;
-#pragma unroll
-          for (int r = 0; r < 2; r++) {
-            if (32 * r >= a.kp) break;
-            uint32_t rh[2][16], rl[2][16];
-#pragma unroll
-            for (int h = 0; h < 2; h++)
-              if (32 * r + 16 * h < a.kp) {
-                tmem_ld16_nowait(taddr + 32 * r + 16 * h, rh[h]);
-                if (BLO && a.sep_lo) tmem_ld16_nowait(taddr + a.kp + 32 * r + 16 * h, rl[h]);
-              }
-            tmem_ld_wait();
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-              tmem_regs_ready(rh[h]);
-              if (BLO && a.sep_lo) tmem_regs_ready(rl[h]);
-            }
-            uint32_t bits = 0;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-              if (32 * r + 16 * h >= a.kp) break;
-#pragma unroll
-              for (int q = 0; q < 4; q++) {
-                const int c4 = 32 * r + 16 * h + 4 * q;
-                const float4 n4 = *reinterpret_cast<const float4*>(snc + c4);
-                const float4 s4 = *reinterpret_cast<const float4*>(scn + c4);
-                const float nn[4] = {n4.x, n4.y, n4.z, n4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                  float x = __uint_as_float(rh[h][4 * q + u]);
-                  if (BLO && a.sep_lo) x += __uint_as_float(rl[h][4 * q + u]);
-                  const float dt = fmaf(-2.0f, x, nxi + nn[u]);
-                  const float sj = nonneg ? fmaxf(x, 0.0f) * a.s_scale : xni * ss[u];
-                  const float e = (a.alpha * sj + a.beta * (nxi + nn[u])) * (1.0f + a.gamma) + a.gamma * fabsf(dt);
-                  bits |= (!(dt - e > hi) ? 1u : 0u) << (16 * h + 4 * q + u);
-                }
-              }
-            }
-            if (r == 0) blo = bits;
-            else bhi = bits;
-          }
-          const uint64_t kmask = a.k >= 64 ? ~0ull : ((1ull << a.k) - 1ull);
-          m0 = ((((uint64_t)bhi) << 32) | blo) & kmask & ~(1ull << bj);
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acce[buf]);
-      } else {
-      // pass 1: screened argmin (first index wins ties)
-      for (int c0 = 0; c0 < a.kp; c0 += 16) {
-        float v[16];
-        tmem_ld16(taddr + c0, v);
-        if (BLO && a.sep_lo) {
-          float w[16];
-          tmem_ld16(taddr + a.kp + c0, w);
-#pragma unroll
-          for (int j = 0; j < 16; j++) v[j] += w[j];
-        }
-#pragma unroll
-        for (int j = 0; j < 16; j++) {
-          const int col = c0 + j;
-          if (col < a.k) {
-            const float dt = fmaf(-2.0f, v[j], nxi + snc[col]);
-            if (dt < best) {
-              best = dt;
-              bj = col;
-              best_dot = v[j];
-            }
+            for (int u = 0; u < 16; u += 2)
+              vmax = max3_f32(vmax, __uint_as_float(rh[h][u]), __uint_as_float(rh[h][u + 1]));
           }
         }
       }
-      // S_j bounds sum_i |x_i c_ij|: |x||c_j| in general, the (inflated) dot product for nonnegative data
-      const float sb = nonneg ? fmaxf(best_dot, 0.0f) * a.s_scale : xni * scn[bj];
-      const float eb = (a.alpha * sb + a.beta * (nxi + snc[bj])) * (1.0f + a.gamma) + a.gamma * fabsf(best);
-      const float hi = best + eb;
-      // pass 2: every other centre whose lower bound reaches the best's upper bound
-      for (int c0 = 0; c0 < a.kp; c0 += 16) {
-        float v[16];
-        tmem_ld16(taddr + c0, v);
-        if (BLO && a.sep_lo) {
-          float w[16];
-          tmem_ld16(taddr + a.kp + c0, w);
+      best = fminf(fminf(b4[0], b4[1]), fminf(b4[2], b4[3]));
+      // S_j bounds sum_i |x_i c_ij|: |x||c_j| in general, the (inflated) dot product
+      // for nonnegative data.  amax: a column's error bound without its share of
+      // |dt|, at the largest S_j and norm (inflated past its own roundings).  hi: the
+      // best column's upper bound; a column above T has its lower bound above hi:
+      // dt (1 - gamma) - amax > hi for dt > T > 0.
+      constexpr float kInfl = 1.0f + 0x1p-18f;
+      const float smax = nonneg ? vmax * a.s_scale : xni * scnmax;
+      const float amax = (a.alpha * smax + a.beta * (nxi + sncmax)) * (1.0f + a.gamma) * kInfl;
+      const float hi = __fadd_ru(__fadd_ru(best, amax), a.gamma * fabsf(best));
+      const float T0 = (hi + amax) * (1.0f + 2.0f * a.gamma) * (1.0f + 0x1p-20f);
+      // finite norms below 2^124 keep every dt finite
+      const bool finite = cta_finite && nxi < 0x1p124f && T0 > 0.0f && T0 < 0x1p127f;
+      const float T = finite ? T0 : __int_as_float(0x7f800000);
+      // Pass 2: the columns up to T, one instruction each: the sign of dt - T', T' the
+      // next value above T.  A row with one such column is decided.
+      const float nt = -__int_as_float(__float_as_int(T) + (finite ? 1 : 0));
+      const f32x2 nt2 = pack2(nt, nt);
+      int near = 0;
+      for (int c0 = 0; c0 < a.kp; c0 += 32) {
+        uint32_t bits = 0;  // the last column at bit 0
+        if (a.kp > 32) columns(c0);  // (otherwise still in rh)
 #pragma unroll
-          for (int j = 0; j < 16; j++) v[j] += w[j];
-        }
+        for (int h = 0; h < 2; h++) {
+          if (c0 + 16 * h >= a.kp) break;
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-          const int col = c0 + j;
-          if (col < a.k && col != bj) {
-            const float dt = fmaf(-2.0f, v[j], nxi + snc[col]);
-            const float sj = nonneg ? fmaxf(v[j], 0.0f) * a.s_scale : xni * scn[col];
-            const float e = (a.alpha * sj + a.beta * (nxi + snc[col])) * (1.0f + a.gamma) + a.gamma * fabsf(dt);
-            if (!(dt - e > hi)) {
-              const uint64_t bit = 1ull << (col & 63);
-              const int w = col >> 6;
-              if (w == 0) m0 |= bit;
-              else if (w == 1) m1 |= bit;
-              else if (w == 2) m2 |= bit;
-              else m3 |= bit;
+          for (int q = 0; q < 4; q++) {
+            float dt[4], cc[4];
+            screen4(c0, h, q, dt, cc);
+#pragma unroll
+            for (int u = 0; u < 4; u += 2) {
+              float e0, e1;
+              unpack2(add2(pack2(dt[u], dt[u + 1]), nt2), e0, e1);
+              bits = __funnelshift_l(__float_as_uint(e0), bits, 1);
+              bits = __funnelshift_l(__float_as_uint(e1), bits, 1);
             }
           }
+        }
+        near += __popc(bits);
+        if (bits) bj = min(c0 + 32, a.kp) - __ffs(bits);
+      }
+      bool found = finite && near == 1;
+      if (__any_sync(0xffffffffu, valid && !found)) {
+        // Pass 3: the first column with the smallest value is the best centre (first
+        // index wins ties, as in a scan; none, a NaN: every centre is a candidate), and
+        // every other column whose own lower bound reaches hi is a candidate.
+        bj = 0;
+        found = false;
+        for (int c0 = 0; c0 < a.kp; c0 += 32) {
+          uint32_t bits = 0, eq = 0;
+          if (a.kp > 32) columns(c0);
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            if (c0 + 16 * h >= a.kp) break;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              float dt[4], cc[4];
+              screen4(c0, h, q, dt, cc);
+              const float4 s4 = *reinterpret_cast<const float4*>(scn + c0 + 16 * h + 4 * q);
+              const float ss[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+              for (int u = 0; u < 4; u++) {
+                const float sj = nonneg ? fmaxf(__uint_as_float(rh[h][4 * q + u]), 0.0f) * a.s_scale : xni * ss[u];
+                const float e = (a.alpha * sj + a.beta * (nxi + cc[u])) * (1.0f + a.gamma) + a.gamma * fabsf(dt[u]);
+                const uint32_t bit = 1u << (16 * h + 4 * q + u);
+                eq |= dt[u] == best ? bit : 0u;
+                bits |= !(dt[u] > T) && !(dt[u] - e > hi) ? bit : 0u;
+              }
+            }
+          }
+          if (!found && eq) {
+            found = true;
+            bj = c0 + __ffs(eq) - 1;
+            bits &= ~(eq & (0u - eq));
+          }
+          if (c0 + 32 > a.k) bits &= c0 < a.k ? (1u << (a.k - c0)) - 1u : 0u;  // (padding columns)
+          const uint64_t word = (uint64_t)bits << (c0 & 32);
+          if (c0 < 64) m0 |= word;
+          else if (c0 < 128) m1 |= word;
+          else if (c0 < 192) m2 |= word;
+          else m3 |= word;
+        }
+        if (!found) {
+          auto all = [&](int c0) { return a.k >= c0 + 64 ? ~0ull : a.k > c0 ? (1ull << (a.k - c0)) - 1ull : 0ull; };
+          m0 = all(0), m1 = all(64), m2 = all(128), m3 = all(192);
         }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acce[buf]);
-      }
       const bool und = (m0 | m1 | m2 | m3) != 0;
       if (a.fused) commit(valid && !und, i, bj, old_lab);  // undecided points: committed by the re-score kernel
       if (valid) {
