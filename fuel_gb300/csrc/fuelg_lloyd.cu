@@ -45,6 +45,9 @@ struct ExactSums;
 ExactSums* exact_sums_new();
 void exact_sums_delete(ExactSums*);
 int exact_sums_init(ExactSums* s, const float* X, int64_t n, int d, int k, cudaStream_t stream);
+bool exact_sums_assigns(int64_t n, int d, int k);
+int exact_sums_assign_step(ExactSums* s, const float* X, const float* from, int order, int32_t* labels, bool first,
+                           bool write_centers, float* centers, int32_t* changed, cudaStream_t stream);
 int exact_sums_step(ExactSums* s, const float* X, const int32_t* lab_new, int32_t* labels, bool first,
                     bool write_centers, float* centers, int32_t* changed, int* dev_status, cudaStream_t stream,
                     const CentrePrep* cp);
@@ -425,6 +428,12 @@ int lloyd_run(const LloydParams& p, LloydResult* r, int* dev_status, cudaStream_
   if (exact) exact_sums_commit_view(es, &scv);
   auto pass = [&](bool first, bool write_centers, int32_t* chg) -> int {
     const bool fused = tc && exact && !first && d <= 1024;
+    const bool small = !tc && exact && exact_sums_assigns(n, d, k);
+    if (small) {
+      if (p.tol > 0 && write_centers)
+        FUELG_CUDA(cudaMemcpyAsync(cold.p, C, sizeof(float) * k * d, cudaMemcpyDeviceToDevice, stream));
+      return exact_sums_assign_step(es, p.X, C, p.order, labels, first, write_centers, C, chg, stream);
+    }
     if (fused) FUELG_TRY(lloyd_tc_pass_fused(p, tc, C, labels, scv, dev_status, stream));
     else FUELG_TRY(assign(first));
     if (p.tol > 0 && write_centers)
