@@ -1523,6 +1523,18 @@ struct DevBuf {
 // range of bytes, aligned for floats, that lies in one allocation of this device.
 constexpr int kDeviceMem = 1, kHereInRange = 2;
 int pointer_kind(const void* ptr, size_t bytes, int dev) {
+  // (through the runtime: the library loads on machines without a driver)
+  using Fn = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Fn attributes = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return (Fn)f;
+  }();
   CUmemorytype type = (CUmemorytype)0;
   unsigned managed = 0;
   int ord = -1;
@@ -1533,7 +1545,15 @@ int pointer_kind(const void* ptr, size_t bytes, int dev) {
                                CU_POINTER_ATTRIBUTE_RANGE_SIZE};
   void* out[5] = {&type, &managed, &ord, &start, &size};
   const CUdeviceptr a = (CUdeviceptr)(uintptr_t)ptr;
-  if (cuPointerGetAttributes(5, at, out, a) != CUDA_SUCCESS || type != CU_MEMORYTYPE_DEVICE || managed) return 0;
+  if (attributes == nullptr) {
+    cudaPointerAttributes pa;
+    if (cudaPointerGetAttributes(&pa, ptr) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return pa.type == cudaMemoryTypeDevice ? kDeviceMem : 0;
+  }
+  if (attributes(5, at, out, a) != CUDA_SUCCESS || type != CU_MEMORYTYPE_DEVICE || managed) return 0;
   const bool here = ord == dev && (a & 3) == 0 && a >= start && bytes <= size && a - start <= size - bytes;
   return kDeviceMem | (here ? kHereInRange : 0);
 }
