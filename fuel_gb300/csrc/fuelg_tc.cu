@@ -21,7 +21,9 @@
 //               per pipeline stage (128-byte swizzle), mbarrier complete_tx
 //   warp 1      TMEM owner and single-thread tcgen05.mma issuer (M=128,
 //               N=kp, K=16 per instruction), tcgen05.commit to free stages
-//   warps 2-5   epilogue: tcgen05.ld of the accumulator rows, screen, write
+//   warps 2-5   epilogue: tcgen05.ld of the accumulator rows, screen, write;
+//               where only one CTA fits an SM, warps 6-9 are a second group, each
+//               with one accumulator
 // Two TMEM accumulators alternate so the epilogue of tile t overlaps the MMAs
 // of tile t+1.  Every mbarrier wait is bounded (globaltimer); on expiry the
 // kernel records DEV_TIMEOUT, stops all roles and still frees its TMEM.
@@ -47,7 +49,6 @@ using namespace tcx;
 namespace {
 
 constexpr int BM = 128;  // points per tile (UMMA M)
-constexpr int kTcThreads = 192;
 
 // Exact re-score of the undecided points: each candidate centre is scored
 // with the reference's own f32 operation order, first minimum wins.  One warp
@@ -188,8 +189,8 @@ struct TcArgs {
 // products; the A lo term of the split form is identically zero).
 constexpr int kBf16 = 0, kSplit = 1, kScaledA = 2;
 
-template <int MODE>
-__global__ void __launch_bounds__(kTcThreads, 2)
+template <int MODE, int GROUPS>
+__global__ void __launch_bounds__(64 + BM * GROUPS, GROUPS == 1 ? 2 : 1)
     lloyd_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmAlo,
                     const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmBlo, TcArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -197,6 +198,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   const uint32_t a_bytes = BM * BK * 2;
   const uint32_t b_bytes = (uint32_t)a.kp * BK * 2;
   constexpr bool ALO = MODE == kSplit, BLO = MODE != kBf16;
+  constexpr int EPI = BM * GROUPS;  // epilogue threads
   const uint32_t stage_bytes = (ALO ? 2u : 1u) * a_bytes + (BLO ? 2u : 1u) * b_bytes;
   // stage layout: A | B | A lo (kSplit) | B lo (kSplit, kScaledA)
   const uint32_t off_alo = a_bytes + b_bytes, off_blo = (ALO ? 2u : 1u) * a_bytes + b_bytes;
@@ -277,7 +279,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   bool cta_finite = true;
   if (warp >= 2) {
     const int kp64 = (a.kp + 63) & ~63;
-    for (int j = threadIdx.x - 64; j < kp64; j += BM) {
+    for (int j = threadIdx.x - 64; j < kp64; j += EPI) {
       // squared norms: the sum of the two halves the centre update wrote
       const float nc2 = j < a.kp ? a.nc[j] + a.nc[a.kp + j] : 0.0f;
       if (j < a.kp) {
@@ -288,7 +290,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       }
       sncd[j] = j < a.k ? nc2 : __int_as_float(0x7f800000);
     }
-    named_bar_sync(1, BM);
+    named_bar_sync(1, EPI);
     // (NaN norms are not finite; a maximum that missed one is then unused)
     for (int j = lane; j < a.k; j += 32) {
       const float s2 = snc[j], c1 = scn[j];
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       if (!mbar_wait(fin, 0, &never)) atomicOr(a.status, DEV_TIMEOUT);
     }
   } else {
-    // epilogue: warps 2..5 -> TMEM lane groups 2,3,0,1
+    // epilogue: warps 2..5 (and 6..9) -> TMEM lane groups 2,3,0,1
     const int g = warp & 3;
     const int row = g * 32 + lane;
     // fused: commit a label (warp-collective; act: this lane has one) --
@@ -435,9 +437,10 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         }
       }
     };
-    int64_t lt = 0;
+    // (two groups: one per accumulator, each with every second tile)
+    int64_t lt = GROUPS == 2 ? (warp - 2) >> 2 : 0;
     const bool nonneg = *a.neg_flag == 0;
-    for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x, lt++) {
+    for (int64_t t = blockIdx.x + lt * gridDim.x; t < ntiles; t += (int64_t)GROUPS * gridDim.x, lt += GROUPS) {
       const uint32_t buf = (uint32_t)(lt & 1), accph = (uint32_t)((lt >> 1) & 1);
       // this point's norms and current label, loaded while the tile's MMAs run
       const int64_t i = t * BM + row;
@@ -457,8 +460,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       // Screen over the TMEM columns, 32 per wait, without branches on a column's
       // value: dt_c = fma(-2, v_c, |x|^2 + |c|^2), +inf for padding columns.
       // (Scans with a branch per column above 64 centres: 20 passes over 100 000 x 64,
-      // k = 200 3.83 -> 1.76 ms, 200 000 x 32, k = 128 4.56 -> 1.99, 76 000 x 784, k =
-      // 250 4.33 -> 2.92; up to 64 centres equal to the tournament tree this replaced,
+      // k = 200 3.83 -> 1.76 ms (1.56 with two groups), 200 000 x 32, k = 128 4.56 -> 1.99 (1.78),
+      // 76 000 x 784, k = 250 4.33 -> 2.92 (2.91); up to 64 centres equal to the tournament tree this replaced,
       // which the row loads and the update kernels bound.  With the best centre's own
       // bound in pass 3, one sweep more, 1 to 4 % slower for 6 to 11 % fewer re-scores.)
       float best = __int_as_float(0x7f800000);
@@ -641,8 +644,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     }
     if (a.fused) {
       // this CTA's histograms into the global ones
-      named_bar_sync(1, BM);
-      for (int j = threadIdx.x - 64; j < a.k; j += BM) {
+      named_bar_sync(1, EPI);
+      for (int j = threadIdx.x - 64; j < a.k; j += EPI) {
         if (h_in[j]) atomicAdd(&a.sc.cin[j], h_in[j]);
         if (h_out[j]) atomicAdd(&a.sc.cout[j], h_out[j]);
       }
@@ -898,6 +901,19 @@ struct TcLloydState {
   CUtensorMap tmA, tmAlo, tmB, tmBlo;
 };
 
+// Epilogue groups: one where two CTAs share an SM, two where one has it alone (more
+// than 64 centres with hi / lo accumulators, 128 without).  20 passes with one group
+// and two: 100 000 x 64, k = 200 1.74 and 1.56 ms; 200 000 x 64, k = 65 1.88 and 1.66; up to
+// 64 centres two CTAs of one group against one of two: 70 000 x 784, k = 64, 100 passes,
+// 5.49 and 6.35 to 6.75.
+static int tc_groups(const TcLloydState* st) { return st->ctas_per_sm == 1 ? 2 : 1; }
+static auto tc_kernel(const TcLloydState* st) {
+  auto pick = [&](auto one, auto two) { return tc_groups(st) == 2 ? two : one; };
+  return st->mode == kScaledA ? pick(lloyd_tc_kernel<kScaledA, 1>, lloyd_tc_kernel<kScaledA, 2>)
+         : st->mode == kSplit ? pick(lloyd_tc_kernel<kSplit, 1>, lloyd_tc_kernel<kSplit, 2>)
+                              : pick(lloyd_tc_kernel<kBf16, 1>, lloyd_tc_kernel<kBf16, 2>);
+}
+
 bool lloyd_tc_supported(int d, int k) { return d >= 32 && k >= 1 && k <= 256; }
 
 int lloyd_tc_prepare(const LloydParams& p, TcLloydState* st, cudaStream_t stream) {
@@ -1008,8 +1024,7 @@ int lloyd_tc_prepare(const LloydParams& p, TcLloydState* st, cudaStream_t stream
   st->tmBlo = st->tmB;
   if (alo) FUELG_TRY(tcx::make_map_bf16(&st->tmAlo, st->xlo.p, st->arows * st->kc, BK, BM));
   if (blo) FUELG_TRY(tcx::make_map_bf16(&st->tmBlo, st->clo.p, st->kp, st->dp, st->kp));
-  auto kern = st->mode == kScaledA ? lloyd_tc_kernel<kScaledA>
-              : st->mode == kSplit ? lloyd_tc_kernel<kSplit> : lloyd_tc_kernel<kBf16>;
+  auto kern = tc_kernel(st);
   FUELG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st->smem));
   return ST_OK;
 }
@@ -1099,9 +1114,8 @@ int tc_pass(const LloydParams& p, TcLloydState* st, const float* centers, bool f
   HotTimer* ht = hot_timer();
   if (ht) ht->begin(stream);
   {
-    auto kern = st->mode == kScaledA ? lloyd_tc_kernel<kScaledA>
-                : st->mode == kSplit ? lloyd_tc_kernel<kSplit> : lloyd_tc_kernel<kBf16>;
-    FUELG_TRY(launch_pdl(kern, dim3(grid), dim3(kTcThreads), st->smem, stream, st->tmA, st->tmAlo, st->tmB,
+    auto kern = tc_kernel(st);
+    FUELG_TRY(launch_pdl(kern, dim3(grid), dim3(64 + BM * tc_groups(st)), st->smem, stream, st->tmA, st->tmAlo, st->tmB,
                          st->tmBlo, a));
   }
   if (ht) ht->end(stream);

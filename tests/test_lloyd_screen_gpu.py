@@ -27,3 +27,16 @@ def test_screen_matches_fp32_tier(gpu, k, d, precision):
     np.testing.assert_array_equal(got.labels, ref.labels)
     np.testing.assert_array_equal(got.centers.view(np.uint32), ref.centers.view(np.uint32))
     assert got.n_iter == ref.n_iter
+
+
+@pytest.mark.parametrize("n", [152 * 128, 152 * 128 + 1, 152 * 128 * 3 + 5])
+@pytest.mark.parametrize("k,precision", [(65, "split_bf16"), (250, "split_bf16"), (200, "bf16"), (40, "split_bf16")])
+def test_screen_several_tiles_per_block(gpu, n, k, precision):
+    """One to four tiles per block, with one epilogue group (k = 40) and two."""
+    rng = np.random.default_rng(n + k)
+    X = (rng.normal(size=(n, 33)) + 3 * rng.integers(-2, 3, size=(n, 1))).astype(np.float32)
+    init = X[rng.permutation(n)[:k]].copy()
+    got = kmeans(X, k=k, variant="lloyd", init=init, max_iter=3, fixed_iters=True, precision=precision)
+    ref = kmeans(X, k=k, variant="lloyd", init=init, max_iter=3, fixed_iters=True, precision="fp32")
+    np.testing.assert_array_equal(got.labels, ref.labels)
+    np.testing.assert_array_equal(got.centers.view(np.uint32), ref.centers.view(np.uint32))
