@@ -128,7 +128,10 @@ __device__ __forceinline__ void commit_body(int bid, int nblk, int32_t* h_in, in
 // the label extraction and the commit took 10.2 + 2.8 + 2.7 + 5.8 us and four launches
 // a pass.
 constexpr int kSmallMaxK = 256, kSmallMaxD = 64;
-constexpr double kSmallWork = 1.6e7;  // n k d
+constexpr double kSmallWork = 1.6e7;    // n k d of assign_commit_kernel
+constexpr double kOnePassWork = 3.2e7;  // n k d of small_pass_kernel
+constexpr int64_t kOnePassSums = 2560;  // k d of small_pass_kernel
+constexpr int kAggCap = 2048;           // 64-bit sums of a block in shared memory (16 KB)
 template <int KIND, int ORDER>
 __global__ void __launch_bounds__(256) assign_commit_kernel(
     const float* __restrict__ X, const float* __restrict__ C, int d, int S, int64_t n, int first, int k,
@@ -424,6 +427,106 @@ __device__ __forceinline__ float mean_elem(unsigned long long* __restrict__ limb
 }
 
 // Hand the change count to the host and reset the per-pass counters.
+// Few sums: a whole pass in one launch.  As assign_commit_kernel, but a changed
+// point's coordinates go straight to the sums -- its S lanes share them, one atomic
+// per 32-bit slice, into the block's own sums where they fit (agg) and those into the
+// global ones at the end -- and the last block to finish (a ticket after a fence: no
+// waiting) makes the means.  Latency bound.  12 passes against assign_commit and the
+// three update launches: 3000 x 10, k = 8 364 -> 301 us; 15 000 x 5, k = 30 499 -> 353;
+// 1 000 000 x 2, k = 3 1392 -> 690.  (Without the blocks' own sums all points of the
+// first pass meet at a few counters: 4917 us there.)
+template <int KIND, int ORDER, int L>
+__global__ void __launch_bounds__(256) small_pass_kernel(
+    const float* __restrict__ X, int d, int S, int64_t n, int first, int k, int e_lo, int write_centers,
+    int agg, float* centers, int32_t* __restrict__ labels, unsigned long long* limbs, int32_t* counts, int32_t* nchg,
+    int32_t* __restrict__ changed, unsigned* __restrict__ done) {
+  __shared__ unsigned long long s_sum[kAggCap];
+  __shared__ int32_t s_cnt[kSmallMaxK];
+  __shared__ int32_t s_chg;
+  __shared__ unsigned s_last;
+  griddep_wait();
+  griddep_launch();
+  for (int j = threadIdx.x; j < k; j += blockDim.x) s_cnt[j] = 0;
+  if (agg)
+    for (int e = threadIdx.x; e < k * d * L; e += blockDim.x) s_sum[e] = 0;
+  if (threadIdx.x == 0) s_chg = 0;
+  __syncthreads();
+  const int s = threadIdx.x & (S - 1);
+  const int per = blockDim.x / S;  // points per block and round
+  auto add = [&](int j, int t, float x, bool out) {
+    const int e = (j * d + t) * L;
+    const unsigned __int128 v = L <= 2 ? (unsigned __int128)fixed_of64(x, e_lo, out) : fixed_of(x, e_lo, out);
+#pragma unroll
+    for (int l = 0; l < L; l++) {
+      const unsigned long long sl = (unsigned long long)((v >> (32 * l)) & 0xffffffffu);
+      if (!sl) continue;
+      if (agg) {
+        // (a 64-bit add in shared memory is a compare-and-swap loop: the low word
+        // and its carry)
+        uint32_t* w = reinterpret_cast<uint32_t*>(s_sum + e + l);
+        if (atomicAdd(w, (uint32_t)sl) > ~(uint32_t)sl) atomicAdd(w + 1, 1u);
+      } else {
+        atomicAdd(limbs + e + l, sl);
+      }
+    }
+  };
+  for (int64_t base0 = (int64_t)blockIdx.x * per; base0 < n; base0 += (int64_t)gridDim.x * per) {
+    const int64_t i = base0 + threadIdx.x / S;
+    uint64_t best = KEY_NONE;
+    int32_t old = -1;
+    const float* x = X + (i < n ? i : 0) * d;
+    if (i < n) {
+      if (!first) old = labels[i];
+      for (int j = s; j < k; j += S) {
+        const uint64_t key = make_key(exact_dist_scalar<KIND, ORDER>(x, centers + (int64_t)j * d, d), (uint32_t)j);
+        best = key < best ? key : best;
+      }
+    }
+    for (int o = S >> 1; o > 0; o >>= 1) {
+      const uint64_t v = __shfl_xor_sync(0xffffffffu, best, o);
+      best = v < best ? v : best;
+    }
+    const int32_t nw = (int32_t)key_idx(best);
+    if (i < n && nw != old) {
+      if (s == 0) {
+        labels[i] = nw;
+        atomicAdd(&s_chg, 1);
+        atomicAdd(&s_cnt[nw], 1);
+        if (old >= 0) atomicAdd(&s_cnt[old], -1);
+      }
+      for (int t = s; t < d; t += S) {
+        const float xv = __ldg(x + t);
+        add(nw, t, xv, false);
+        if (old >= 0) add(old, t, xv, true);
+      }
+    }
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < k; j += blockDim.x)
+    if (s_cnt[j]) atomicAdd(&counts[j], s_cnt[j]);
+  if (agg && s_chg)
+    for (int e = threadIdx.x; e < k * d * L; e += blockDim.x)
+      if (s_sum[e]) atomicAdd(limbs + e, s_sum[e]);
+  if (threadIdx.x == 0 && s_chg) atomicAdd(nchg, s_chg);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1 ? 1u : 0u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int e = threadIdx.x; e < k * d; e += blockDim.x) {
+    unsigned long long lv[L];
+#pragma unroll
+    for (int l = 0; l < L; l++) lv[l] = __ldcg(limbs + (int64_t)e * L + l);
+    mean_of<L>(limbs + (int64_t)e * L, lv, __ldcg(counts + e / d), e_lo, centers + e, centers[e], write_centers);
+  }
+  if (threadIdx.x == 0) {
+    *changed = __ldcg(nchg);
+    *nchg = 0;
+    *done = 0;
+  }
+}
+
 __device__ __forceinline__ void mean_handoff(int bid, int nblk, int32_t* __restrict__ nchg,
                                              int32_t* __restrict__ changed, int32_t* __restrict__ zero4k, int nzero) {
   if (bid == 0 && threadIdx.x == 0) {
@@ -679,12 +782,16 @@ int exact_sums_step(ExactSums* s, const float* X, const int32_t* lab_new, int32_
 
 // exact_sums_step with the assignment itself in the same kernel (assign_commit_kernel):
 // labels become the nearest of `from` by the exact arithmetic.
-// Up to n k d = 1.6 10^7 it is faster (12 passes: 3000 x 10, k = 8 501 -> 367 us; 2000 x 30,
-// k = 32 653 -> 398; 15 000 x 31, k = 32 699 -> 566; 400 000 x 8, k = 4 949 -> 907), above it
-// the tiled scan, which reads rows and centres once per block, is (200 000 x 8, k = 16 776
-// for 907; 30 000 x 24, k = 64 683 for 709).
+// Up to n k d = 1.6 10^7 it is faster (12 passes: 2000 x 30, k = 32 653 -> 388 us; 5000 x 10,
+// k = 250 870 -> 624), above it the tiled scan, which reads rows and centres once per
+// block, is (200 000 x 8, k = 16 776 for 907; 30 000 x 24, k = 64 683 for 709).  With the
+// whole pass in one launch (small_pass_kernel) the line is 3.2 10^7 (200 000 x 8, k = 16
+// 775 and 774; 100 000 x 10, k = 32 722 -> 582; 30 000 x 24, k = 64 681 for 701), up to
+// k d = 2560 means, which one block makes (5000 x 10, k = 250 624 -> 491; 1000 x 31, k = 256
+// 557 for 924).
 bool exact_sums_assigns(int64_t n, int d, int k) {
-  return k <= kSmallMaxK && d <= kSmallMaxD && (double)n * k * d <= kSmallWork;
+  return k <= kSmallMaxK && d <= kSmallMaxD &&
+         (double)n * k * d <= (k * d <= kOnePassSums ? kOnePassWork : kSmallWork);
 }
 
 int exact_sums_assign_step(ExactSums* s, const float* X, const float* from, int order, int32_t* labels, bool first,
@@ -697,6 +804,31 @@ int exact_sums_assign_step(ExactSums* s, const float* X, const float* from, int 
   int S = 1;
   while (S < 32 && S < k && 2 * S * n <= (int64_t)152 * 2048) S *= 2;
   const unsigned blocks = (unsigned)std::min<int64_t>((n * S + 255) / 256, 8 * 152);
+  if ((int64_t)k * s->d <= kOnePassSums) {
+    const int agg = (int64_t)k * s->d * s->L <= kAggCap ? 1 : 0;
+    HotTimer* ht = hot_timer();
+    if (ht) ht->begin(stream);
+    auto run = [&](auto kern) {
+      return launch_pdl(kern, dim3(blocks), dim3(256), 0, stream, X, s->d, S, n, first ? 1 : 0, k, s->e_lo,
+                        write_centers ? 1 : 0, agg, centers, labels, s->limbs.as<unsigned long long>(),
+                        s->counts.as<int32_t>(), s->nchg.as<int32_t>(), changed, s->done.as<unsigned>());
+    };
+    auto pick = [&](auto Lc) {
+      constexpr int LL = decltype(Lc)::value;
+      return order == ORDER_X86 ? (first ? run(small_pass_kernel<KIND_PAIRWISE, ORDER_X86, LL>)
+                                         : run(small_pass_kernel<KIND_SQDIST, ORDER_X86, LL>))
+                                : (first ? run(small_pass_kernel<KIND_PAIRWISE, ORDER_ARM, LL>)
+                                         : run(small_pass_kernel<KIND_SQDIST, ORDER_ARM, LL>));
+    };
+    switch (s->L) {
+      case 1: FUELG_TRY(pick(std::integral_constant<int, 1>())); break;
+      case 2: FUELG_TRY(pick(std::integral_constant<int, 2>())); break;
+      case 3: FUELG_TRY(pick(std::integral_constant<int, 3>())); break;
+      default: FUELG_TRY(pick(std::integral_constant<int, 4>())); break;
+    }
+    if (ht) ht->end(stream);
+    return ST_OK;
+  }
   auto go = [&](auto kern) {
     return launch_pdl(kern, dim3(blocks), dim3(256), 0, stream, X, from, s->d, S, n, first ? 1 : 0, k, labels,
                       s->chg_i.as<int32_t>(), s->chg_old.as<int32_t>(), s->chg_new.as<int32_t>(),
