@@ -88,6 +88,7 @@ struct KnnTcArgs {
   float xmax_n2;     // max |x|^2 over the index (filter slack)
   uint64_t* lists;     // [CTA][QB][kKeep + 2 kLog]: kept keys and logs of the rows a CTA works on
   uint64_t* out_keys;  // [piece][QB][kout]: each piece's kept keys
+  int spread;          // one block: the epilogue warps its queries are dealt to (spread_query), or 0
   // Work decomposition: CTA c works through pieces [cta_pb[c], cta_pb[c+1]);
   // piece p = query block piece_qb[p] against index tiles [piece_t0[p], piece_t1[p]).
   const int32_t* piece_qb;
@@ -146,6 +147,11 @@ __global__ void __launch_bounds__(256) sort_rows_kernel(uint64_t* __restrict__ k
   else if (last <= 3) sort_row<4>(kr, kk2, lane);
   else sort_row<8>(kr, kk2, lane);
 }
+
+// The query of row r where the queries of one block are dealt to `warps` epilogue
+// warps (four: one half, or all eight), each an equal share: limits after the warm-up
+// and lists out are work of 4 to 6 us a row, one row at a time.
+__device__ __forceinline__ int spread_query(int r, int warps) { return (r & 31) * warps + (r >> 5); }
 
 constexpr int kMaxSplits = 160;
 
@@ -480,6 +486,11 @@ __device__ __forceinline__ int warm_tiles(int tiles, int need, int* g) {
   *g = 1 << lg;
   return tiles >= 2 && ((128 * w) >> lg) >= need + need / 4 ? w : 0;
 }
+// Whether the block of queries from q0 on has rows in its second half.
+__device__ __forceinline__ bool second_half(const KnnTcArgs& a, int64_t q0) {
+  return a.spread ? a.spread == 8 : q0 + QM < a.m;
+}
+
 // The need of piece p: its rank, or kk where a block is one piece.
 __device__ __forceinline__ int piece_need(const KnnTcArgs& a, int p) {
   if (a.pub == nullptr) return a.kk2;
@@ -604,7 +615,7 @@ __global__ void __launch_bounds__(kThreadsKT, 1)
     for (int p = pb; ok && p < pe; p++) {
       const int t0 = a.piece_t0[p], t1 = a.piece_t1[p];
       const int q0 = a.piece_qb[p] * QB;
-      for (int h = 0; h < 2 && a.ss && q0 + h * QM < a.m; h++) {
+      for (int h = 0; h < 2 && a.ss && (h == 0 || second_half(a, q0)); h++) {
         // the half's query operand, once the last piece's products have read theirs
         ok = loads_a[h] == 0 || mbar_wait(&aempty[h], (uint32_t)((loads_a[h] - 1) & 1), abort_flag, a.wait_ns);
         ok = __all_sync(0xffffffffu, ok);
@@ -681,7 +692,7 @@ __global__ void __launch_bounds__(kThreadsKT, 1)
     bool ok = true;
     for (int p = pb; ok && p < pe; p++) {
       const int li = p - pb;
-      const int nh = (int64_t)a.piece_qb[p] * QB + QM < a.m ? 2 : 1;  // halves with query rows
+      const int nh = second_half(a, (int64_t)a.piece_qb[p] * QB) ? 2 : 1;  // halves with query rows
       int g;
       const int tiles = a.piece_t1[p] - a.piece_t0[p];
       const int ntile = tiles + warm_tiles(tiles, piece_need(a, p), &g);
@@ -774,11 +785,13 @@ __global__ void __launch_bounds__(kThreadsKT, 1)
     for (int p = pb; alive && p < pe; p++) {
       const int64_t q0 = (int64_t)a.piece_qb[p] * QB;
       const int64_t t0 = a.piece_t0[p], t1 = a.piece_t1[p];
-      const int nh = q0 + QM < a.m ? 2 : 1;
+      const int nh = second_half(a, q0) ? 2 : 1;
       int wg;
       const int warm = warm_tiles((int)(t1 - t0), piece_need(a, p), &wg);
       if (half >= nh) continue;
-      const int64_t qi = q0 + row;
+      const int64_t qi = a.spread ? spread_query(row, a.spread) : q0 + row;
+      // this warp's rows with a query (may be <= 0)
+      const int64_t rows_left = a.spread ? (a.m + a.spread - 1 - (half * 4 + g)) / a.spread : a.m - (q0 + half * QM + g * 32);
       const bool valid = qi < a.m;
       {
         // (!ss) this row's operand into TMEM: the products that read the last
@@ -898,8 +911,7 @@ __global__ void __launch_bounds__(kThreadsKT, 1)
       }
       if (!alive) break;
       if (warm > 0) {
-        const int64_t left = a.m - (q0 + half * QM + g * 32);
-        warm_limits(a, lists_w, nv, (int)(left < 32 ? (left > 0 ? left : 0) : 32), half * QM + g * 32, p, s_tau, s_thr,
+        warm_limits(a, lists_w, nv, (int)(rows_left < 32 ? (rows_left > 0 ? rows_left : 0) : 32), half * QM + g * 32, p, s_tau, s_thr,
                     s_nq, s_kk, s_rank, lane);
       }
       for (int i = 0; i < tiles; i++) {
@@ -982,11 +994,11 @@ __global__ void __launch_bounds__(kThreadsKT, 1)
       __syncwarp();
       // kept keys out, one query at a time per warp: a sorted list, or (kk > 32)
       // the kept keys and what is left in the log, unsorted; slots past them are
-      // KEY_NONE.  Piece p's lists sit at rows [p*QB, p*QB + QB) of the output.
+      // KEY_NONE.  Piece p's lists sit at rows [p*QB, p*QB + QB) of the output, in
+      // query order.
       constexpr int NK = kKeep / 32, NL = kLog / 32;
       uint64_t nkey[NK];
       uint2 nent[NL];
-      const int64_t rows_left = a.m - (q0 + half * QM + g * 32);
       const int rows = (int)(rows_left < 32 ? rows_left : 32);  // (may be <= 0)
       auto fetch = [&](int src) {  // a row's kept keys and what is left in its log
         const uint64_t* list = lists_w + src * qstride;
@@ -1008,7 +1020,7 @@ __global__ void __launch_bounds__(kThreadsKT, 1)
         const int sbuf = __shfl_sync(0xffffffffu, buf, src);
         const int skk = s_kk[r];
         uint64_t* list = lists_w + src * qstride;
-        uint64_t* to = a.out_keys + ((size_t)p * QB + r) * a.kout;
+        uint64_t* to = a.out_keys + ((size_t)p * QB + (a.spread ? spread_query(r, a.spread) : r)) * a.kout;
         uint64_t key[NK], add[NL];
         const uint64_t stau = s_tau[r];
         const float snq = s_nq[r];
@@ -1083,14 +1095,15 @@ __global__ void __launch_bounds__(kThreadsKT, 1)
 template <bool F16>
 __global__ void knn_prep_kernel(const float* __restrict__ X, int64_t rows, int64_t rows_pad, int d, int dp,
                                 void* __restrict__ out, __nv_bfloat16* __restrict__ out_lo,
-                                float* __restrict__ n2, int* __restrict__ flags) {
+                                float* __restrict__ n2, int* __restrict__ flags, int spread) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   int bad = 0;
   float vmax = 0.0f;
   for (int64_t r = (int64_t)blockIdx.x * nw + warp; r < rows_pad; r += (int64_t)gridDim.x * nw) {
+    const int64_t src = spread ? spread_query((int)r, spread) : r;
     float acc = 0.0f;
     for (int c = lane; c < dp; c += 32) {
-      const float x = (r < rows && c < d) ? __ldg(X + r * d + c) : 0.0f;
+      const float x = (src < rows && c < d) ? __ldg(X + src * d + c) : 0.0f;
       if (F16) {
         static_cast<__half*>(out)[r * dp + c] = __float2half_rn(x);
       } else {
@@ -1104,7 +1117,7 @@ __global__ void knn_prep_kernel(const float* __restrict__ X, int64_t rows, int64
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (lane == 0) n2[r] = acc;
+    if (lane == 0) n2[src] = acc;
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
@@ -1325,7 +1338,7 @@ int knn_tc_index_build(const float* X32, int64_t n, int d, cudaStream_t stream, 
   FUELG_TRY(flags.alloc(sizeof(int) * 2, stream));
   FUELG_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(int) * 2, stream));
   knn_prep_kernel<false><<<8 * 152, 256, 0, stream>>>(X32, n, t->npad, d, t->dp, t->xb, nullptr, t->xn2,
-                                                      flags.as<int>());
+                                                      flags.as<int>(), 0);
   ::fuelg::note_launch();
   FUELG_CUDA(cudaGetLastError());
   int hf[2];
@@ -1355,7 +1368,7 @@ int knn_tc_index_add_lo(TcIndex* t, const float* X32, cudaStream_t stream) {
   FUELG_TRY(n2.alloc(sizeof(float) * t->npad, stream));
   FUELG_TRY(flags.alloc(sizeof(int) * 2, stream));
   knn_prep_kernel<false><<<8 * 152, 256, 0, stream>>>(X32, t->n, t->npad, t->d, t->dp, hi.as<__nv_bfloat16>(),
-                                                      t->xlo, n2.as<float>(), flags.as<int>());
+                                                      t->xlo, n2.as<float>(), flags.as<int>(), 0);
   ::fuelg::note_launch();
   FUELG_CUDA(cudaGetLastError());
   FUELG_TRY(make_map_bf16(&t->tmXlo, t->xlo, t->npad, t->dp, XN));
@@ -1374,7 +1387,7 @@ int knn_tc_index_add_f16(TcIndex* t, const float* X32, cudaStream_t stream) {
   FUELG_TRY(n2.alloc(sizeof(float) * t->npad, stream));
   FUELG_TRY(flags.alloc(sizeof(int) * 2, stream));
   knn_prep_kernel<true><<<8 * 152, 256, 0, stream>>>(X32, t->n, t->npad, t->d, t->dp, t->xh, nullptr,
-                                                     n2.as<float>(), flags.as<int>());
+                                                     n2.as<float>(), flags.as<int>(), 0);
   ::fuelg::note_launch();
   FUELG_CUDA(cudaGetLastError());
   FUELG_TRY(make_map_bf16(&t->tmXh, t->xh, t->npad, t->dp, XN));  // 2-byte elements: same box geometry
@@ -1394,7 +1407,13 @@ int knn_tc_topk(const TcIndex* ti, const float* Q32, int64_t m, const float* X32
     return ST_ENOTSUP;
   }
   const int kc = dp / BK;
-  const int64_t mpad = ((m + QM - 1) / QM) * QM;
+  // One block's queries are dealt to the epilogue warps: to all eight where that saves
+  // more than the second half's products and tests cost.  Kernel, us, 2 10^6 x 96, k = 10,
+  // rows in order / four / eight warps: FP16 16 queries 178 / 125 / -, 32 253 / 146 / 138,
+  // 128 281 / 284 / 214; split BF16, three products, 32 328 / 223 / 263, 64 353 / 269 / 288,
+  // 128 366 / 368 / 339.  200 000 x 128, 32 queries: the call 315 -> 199.
+  const int spread = m > QB ? 0 : m > (tier == TC_SPLIT ? 64 : 16) ? 8 : 4;
+  const int64_t mpad = spread == 8 ? QB : ((m + QM - 1) / QM) * QM;
   const bool f16 = tier == TC_F16;
   int split = tier == TC_SPLIT ? 1 : 0;
   if (split && !ti->xlo) {
@@ -1413,11 +1432,11 @@ int knn_tc_topk(const TcIndex* ti, const float* Q32, int64_t m, const float* X32
   FUELG_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(int) * 2, stream));
   if (f16)
     knn_prep_kernel<true><<<8 * 152, 256, 0, stream>>>(Q32, m, mpad, d, dp, qb.p, nullptr, qn2.as<float>(),
-                                                       flags.as<int>());
+                                                       flags.as<int>(), spread);
   else
     knn_prep_kernel<false><<<8 * 152, 256, 0, stream>>>(Q32, m, mpad, d, dp, qb.p,
                                                         split ? qlo.as<__nv_bfloat16>() : nullptr, qn2.as<float>(),
-                                                        flags.as<int>());
+                                                        flags.as<int>(), spread);
   ::fuelg::note_launch();
   FUELG_CUDA(cudaGetLastError());
   int hf[2];
@@ -1604,6 +1623,7 @@ int knn_tc_topk(const TcIndex* ti, const float* Q32, int64_t m, const float* X32
     a.margin_mode = mmode;
     a.exact = exact ? 1 : 0;
     a.split = split;
+    a.spread = spread;
     a.stages = stages;
     a.qn2 = qn2.as<float>() + b0;
     a.xmax_n2 = xmax_n2;
