@@ -852,8 +852,12 @@ int exact_range(const ExactScanParams& p, float radius, int exclude_self, int64_
     FUELG_CUDA(cudaMemsetAsync(*d_off, 0, sizeof(int64_t) * (p.m + 1), stream));
     return ST_OK;
   }
-  if (p.kind == KIND_KNN && tile_range_supported(p.d))
-    return tile_range(p, radius, exclude_self, *d_off, d_idx, d_dist, total, stream, radii, passes);
+  if (p.kind == KIND_KNN && tile_range_supported(p.d)) {
+    const int rc = tile_range(p, radius, exclude_self, *d_off, d_idx, d_dist, total, stream, radii, passes);
+    // (without room for the slots: the two passes below, which need none)
+    if (rc != ST_ENOMEM || *passes > 0) return rc;
+    cudaGetLastError();
+  }
   Plan pl;
   FUELG_TRY(make_plan(p, true, scan_np(p.kind, p.order), &pl));
   const int S = pl.S_grid * pl.ws;
