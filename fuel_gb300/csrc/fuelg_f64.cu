@@ -294,8 +294,10 @@ __global__ void __launch_bounds__(kT) knn64_finish_kernel(const double* __restri
 // Rows shifted by the index's first row (a common offset costs the rounded
 // copies no bits; coordinates that are not finite there shift by 0) and rounded
 // to f32.  err[r]: a bound on |row - copy| in the Euclidean norm; vint[r]: the
-// largest |value| of a copy whose values are all integers, else +inf.  all[0]:
-// the largest err (as bits of a double), all[1]: the largest vint (f32 bits).
+// largest |value| of a copy whose values are all integers and the row's exact
+// shifted values, else +inf (100 - 7.000000000000001 rounds to 93 and 1 - 1e-20 to 1:
+// such copies tie where the rows differ).  all[0]: the largest err (as bits of a
+// double), all[1]: the largest vint (f32 bits).
 __global__ void __launch_bounds__(kT) narrow64_kernel(const double* __restrict__ X, int64_t rows, int d,
                                                       const double* __restrict__ centre, float* __restrict__ out,
                                                       double* __restrict__ err, float* __restrict__ vint,
@@ -308,13 +310,16 @@ __global__ void __launch_bounds__(kT) narrow64_kernel(const double* __restrict__
     double e2 = 0.0;
     float vm = 0.0f;
     for (int c = lane; c < d; c += 32) {
-      const double c0 = centre[c];
-      const double v = isfinite(c0) ? X[r * d + c] - c0 : X[r * d + c];
+      const double x = X[r * d + c], c0 = isfinite(centre[c]) ? centre[c] : 0.0;
+      const double v = __dsub_rn(x, c0);
+      // what the subtraction rounded away (the two-sum of x and -c0; NaN past the range)
+      const double t = __dsub_rn(v, x);
+      const double lost = __dsub_rn(__dsub_rn(x, __dsub_rn(v, t)), __dadd_rn(c0, t));
       const float f = __double2float_rn(v);
       out[r * d + c] = f;
       const double e = fabs(v - (double)f) + 1.2e-16 * fabs(v);  // and the shift's own rounding
       e2 = fma(e, e, e2);
-      vm = f == rintf(f) && v == (double)f ? fmaxf(vm, fabsf(f)) : __int_as_float(0x7f800000);
+      vm = f == rintf(f) && v == (double)f && lost == 0.0 ? fmaxf(vm, fabsf(f)) : __int_as_float(0x7f800000);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -344,8 +349,9 @@ __global__ void __launch_bounds__(kT) narrow64_kernel(const double* __restrict__
 // copies' distance times at most 1 + gamma), so its copies are at least
 // sqrt(D_last (1 - gamma)) apart and it is at least that less the two rounding
 // errors from the query; its f64 distance, computed with relative error g64, must
-// exceed the kk-th candidate's.  Where every value is an integer and every partial
-// sum below 2^24, the screened distances are exact and the list is final.
+// exceed the kk-th candidate's.  Where the copies are the exact shifted values, all of
+// them integers, and every partial sum is at most 2^24, the screened distances are
+// exact and the list is final.
 template <int ORDER>
 __global__ void __launch_bounds__(kT) rescore64_kernel(const double* __restrict__ X, const double* __restrict__ Q,
                                                        int64_t m, int64_t q0, int64_t n, int d,
