@@ -599,12 +599,17 @@ __global__ void __launch_bounds__(64 + BM * GROUPS, GROUPS == 1 ? 2 : 1)
               }
             }
           }
+          if (c0 + 32 > a.k) {
+            // padding columns: their +inf is the smallest value too where all others are NaN
+            const uint32_t real = c0 < a.k ? (1u << (a.k - c0)) - 1u : 0u;
+            eq &= real;
+            bits &= real;
+          }
           if (!found && eq) {
             found = true;
             bj = c0 + __ffs(eq) - 1;
             bits &= ~(eq & (0u - eq));
           }
-          if (c0 + 32 > a.k) bits &= c0 < a.k ? (1u << (a.k - c0)) - 1u : 0u;  // (padding columns)
           const uint64_t word = (uint64_t)bits << (c0 & 32);
           if (c0 < 64) m0 |= word;
           else if (c0 < 128) m1 |= word;
