@@ -76,12 +76,13 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
   int polled = 0, stop = 0;
 
   // lane 0: row r's new limit from its kk-th key (never above what other runs of
-  // the query have found)
+  // the query have found).  gthr has m words: rows past m, which keep index rows of
+  // zeros (see below), share no limit.
   auto set_limit = [&](int r, int64_t q, uint64_t tau) {
     if (tau == KEY_NONE) return;
     const unsigned lim = tile_limit_bits(key_dist(tau), a.metric);
     s_thr[r] = min(s_thr[r], lim);
-    if (a.gthr != nullptr) atomicMin(a.gthr + q, lim);
+    if (a.gthr != nullptr && q < a.m) atomicMin(a.gthr + q, lim);
   };
   // folds row j's log into its kept keys (whole warp)
   auto flush = [&](int j, int64_t q0) {
@@ -111,7 +112,8 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
       tile_stage(xT + u * xtile, kTilePS, a.B, (x_first + u) * kTileP, kTileP, a.n, a.d, a.nb);
     if (lane < kTileQ) {
       const int r = warp * kTileQ + lane;
-      // (rows past m are never written: only exact zeros enter them)
+      // (rows past m: their query is all zeros, so index rows of zeros are kept for
+      // them; nothing of theirs is written out)
       s_thr[r] = q0 + r >= a.m ? 0u : a.gthr != nullptr ? *((volatile unsigned*)a.gthr + q0 + r) : 0xffffffffu;
       if (!SMALL) {
         s_cnt[r] = s_len[r] = 0;
