@@ -546,7 +546,7 @@ int index_topk(fuelg_index* ix, const float* Q, int64_t m, int kk, int precision
       rc = knn_tc_topk(ix->tc, Q, m, ix->X, kk, ix->order, ix->metric, tier, keys, dstat, s, rescored, &exact);
     if (rc != ST_OK && rc != ST_ENOTSUP) return rc;
     if (rc == ST_OK) {
-      // integer data run the exact one-product screen whatever the split request
+      // integers that screen exactly take the one-product form whatever the split request
       *used = tier == TC_F16 ? FUELG_PREC_F16 : (tier == TC_SPLIT && !exact) ? FUELG_PREC_SPLIT_BF16 : FUELG_PREC_BF16;
       return ST_OK;
     }

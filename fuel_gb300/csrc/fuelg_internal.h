@@ -263,15 +263,15 @@ struct TcIndex;
 int knn_tc_index_build(const float* X32, int64_t n, int d, cudaStream_t stream, TcIndex** out);
 void knn_tc_index_free(TcIndex* t);
 // Value class of an index's data, which decides the cheapest exact tier:
-// integers with |v| <= 256 (the BF16 screen is exact), values within the FP16
-// range, or wider values.
+// integers with |v| <= 256 (held exactly by BF16; the screen itself is exact where
+// sums cannot round), values within the FP16 range, or wider values.
 constexpr int TC_CLASS_INTEGER = 0, TC_CLASS_F16_RANGE = 1, TC_CLASS_WIDE = 2;
 int knn_tc_index_class(const TcIndex* t);
 int knn_tc_index_add_lo(TcIndex* t, const float* X32, cudaStream_t stream);
 // FP16 copy of the index; ST_ENOTSUP when a value lies outside the FP16 range.
 int knn_tc_index_add_f16(TcIndex* t, const float* X32, cudaStream_t stream);
-// tier: TC_BF16 / TC_SPLIT / TC_F16 operands; integer data whose BF16 screen
-// is exact always use BF16 (no margin, no re-score); FP16 falls back to the
+// tier: TC_BF16 / TC_SPLIT / TC_F16 operands; integer data whose one-product
+// screen is exact use one product (no margin, no re-score); FP16 falls back to the
 // split tier when the queries leave the FP16 range.  row_k (device, m entries, or
 // nullptr): a smaller k per query row -- row q's first row_k[q] keys (of the
 // kk per row written) are its exact top row_k[q]; the rest are unspecified.

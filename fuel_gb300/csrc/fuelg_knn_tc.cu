@@ -21,9 +21,9 @@
 // epilogue; selecting in the epilogue warps stalled both halves' accumulators; a
 // larger unrolled epilogue ran into instruction-cache misses.
 //
-// Exact mode: when every value of the index and the queries is an integer of
-// magnitude <= 256 and 2 d V^2 < 2^24, every BF16 product, every FP32 partial
-// sum (in halves, below 2^23) and D~ itself are exact, D~ an integer below 2^24 --
+// Exact mode (exact_screen): when every value of the index and the queries is an
+// integer of magnitude <= 256 and small enough, every BF16 product, every FP32 partial
+// sum (in halves, at most 2^23) and D~ itself are exact, D~ an integer of at most 2^24 --
 // D~ then IS fuel's f32 distance (src/distance/squared_euclidean.rs sums the same
 // exact integers), whatever the summation order, and the screen keys are final.
 // Otherwise the kk2 = kk + margin best screened keys are re-scored with the
@@ -1094,8 +1094,9 @@ __global__ void __launch_bounds__(kThreadsKT, 1)
 }
 
 // Rows -> BF16 copy padded to dp columns and rows_pad rows (zeros), |row|^2 in
-// FP32, plus an integer-data census: flags[0] |= non-integer or |v| > 256,
-// flags[1] = max |v| (as float bits; non-negative so integer order works).
+// FP32, plus an integer-data census: flags[0] |= 1 for a non-integer or |v| > 256, 2
+// for a negative value, flags[1] = max |v| (as float bits; non-negative so integer
+// order works).
 template <bool F16>
 __global__ void knn_prep_kernel(const float* __restrict__ X, int64_t rows, int64_t rows_pad, int d, int dp,
                                 void* __restrict__ out, __nv_bfloat16* __restrict__ out_lo,
@@ -1116,7 +1117,8 @@ __global__ void knn_prep_kernel(const float* __restrict__ X, int64_t rows, int64
         if (out_lo) out_lo[r * dp + c] = __float2bfloat16_rn(x - __bfloat162float(hi));
       }
       acc = fmaf(x, x, acc);
-      if (x != rintf(x) || fabsf(x) > 256.0f) bad = 1;
+      if (x != rintf(x) || fabsf(x) > 256.0f) bad |= 1;
+      if (x < 0.0f) bad |= 2;
       vmax = fmaxf(vmax, fabsf(x));
     }
 #pragma unroll
@@ -1129,7 +1131,7 @@ __global__ void knn_prep_kernel(const float* __restrict__ X, int64_t rows, int64
     vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, off));
   }
   if (lane == 0) {
-    if (bad) atomicOr(&flags[0], 1);
+    if (bad) atomicOr(&flags[0], bad);
     atomicMax(&flags[1], __float_as_int(vmax));
   }
 }
@@ -1278,6 +1280,17 @@ int sort_and_merge_runs(uint64_t* lists, int64_t m, int qm, int64_t nt, int64_t 
 namespace {
 // Shared memory of knn_tc_kernel beside the query chunks and the index tiles.
 constexpr size_t kFixedSmem = 1024 + kNormBytes + 8 * (2 * kMaxStages + 16) + 16 + QB * 36 + 16;
+// Whether the screened distances of integers up to qmax and xmax in magnitude, in d
+// dimensions (dp with padding), are fuel's f32 distances: partial sums and norms are
+// exact below 2 dp V^2 < 2^24, V the larger, and so is |q - x|^2 <= d V^2 where no value
+// is negative.  With both signs it can reach d (qmax + xmax)^2, up to 4 d V^2: fuel's sums
+// round once they pass 2^24, in an order that D~ does not follow (d = 128, values of
+// 255 and -254: a third of the distances differ).  Up to 2^24 nothing rounds: the
+// products' sums in halves stay within (qmax + xmax)^2 d / 2.
+bool exact_screen(int d, int dp, double qmax, double xmax, bool negative) {
+  const double v = std::max(qmax, xmax);
+  return 2.0 * dp * v * v < 16777216.0 && (!negative || d * (qmax + xmax) * (qmax + xmax) <= 16777216.0);
+}
 // TMEM columns of one half's query operand: two 16-bit values per column.
 int query_cols(int d, int split) { return (split ? 2 : 1) * ((d + BK - 1) / BK) * (BK / 2); }
 int margin_mode_of(int tier) { return tier == TC_F16 ? 2 : 1; }
@@ -1303,6 +1316,7 @@ struct TcIndex {
   __half* xh = nullptr;         // [npad, dp] FP16 (FP16 tier; built on first use)
   float* xn2 = nullptr;         // [npad] FP32 |x|^2 (padded rows 0)
   bool integer = false;         // every value an integer with |v| <= 256
+  bool negative = false;        // some value below 0
   float vmax = 0.0f;            // max |v|
   float xmax_n2 = 0.0f;         // max |x|^2
   uint16_t* xnorm = nullptr;    // [npad, 16] |x|^2 / 2 as three BF16 parts, then zeros
@@ -1350,7 +1364,8 @@ int knn_tc_index_build(const float* X32, int64_t n, int d, cudaStream_t stream, 
   std::vector<float> h((size_t)t->npad);
   FUELG_CUDA(cudaMemcpyAsync(h.data(), t->xn2, sizeof(float) * t->npad, cudaMemcpyDeviceToHost, stream));
   FUELG_CUDA(cudaStreamSynchronize(stream));
-  t->integer = hf[0] == 0;
+  t->integer = (hf[0] & 1) == 0;
+  t->negative = (hf[0] & 2) != 0;
   memcpy(&t->vmax, &hf[1], sizeof(float));
   for (float v : h) t->xmax_n2 = std::max(t->xmax_n2, v);
   norm_parts_kernel<<<(unsigned)((t->npad + 255) / 256), 256, 0, stream>>>(t->xn2, t->npad, t->xnorm);
@@ -1452,9 +1467,8 @@ int knn_tc_topk(const TcIndex* ti, const float* Q32, int64_t m, const float* X32
     set_error("query values exceed the FP16 range (max |q| = %g)", (double)qmax);
     return ST_ENOTSUP;
   }
-  const float vmax = std::max(qmax, ti->vmax);
-  const bool integer = hf[0] == 0 && ti->integer;
-  const bool exact = integer && 2.0 * dp * (double)vmax * vmax < 16777216.0;
+  const bool integer = (hf[0] & 1) == 0 && ti->integer;
+  const bool exact = integer && exact_screen(d, dp, qmax, ti->vmax, (hf[0] & 2) != 0 || ti->negative);
   *exact_out = exact ? 1 : 0;
   if (exact) split = 0;  // integer data: the one-product screen (BF16 or FP16) is already exact
   // screened keys kept per query: exact sqeuclidean needs none extra
@@ -1584,7 +1598,7 @@ int knn_tc_topk(const TcIndex* ti, const float* Q32, int64_t m, const float* X32
   auto kern = knn_tc_kernel;
   // (one limit for every shape: calls on other threads may set it at the same time)
   FUELG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemPerCta));
-  // integer data aside, keep the error-bound constants of the Lloyd screen
+  // exact screens aside, the error-bound constants of the Lloyd screen
   const double u8 = std::ldexp(1.0, -8), u23 = std::ldexp(1.0, -23), u24 = std::ldexp(1.0, -24);
   // operand rounding (2u + u^2 per BF16 product with u = 2^-8; 3.01 * 2^-16
   // with hi + lo; u = 2^-11 per FP16 value in the normal range) plus FP32
@@ -1592,8 +1606,10 @@ int knn_tc_topk(const TcIndex* ti, const float* Q32, int64_t m, const float* X32
   // 2^-14 round with an absolute error of at most 2^-25 instead: the distance
   // (2 q.x) takes 2^-24 (|q|_1 + |x|_1) <= 2^-24 sqrt(dp) (|q| + |x|) more.
   const double u11 = std::ldexp(1.0, -11);
-  // (the norm step adds kNB products, the last ones, at the size of both sums)
-  const double rel = split ? 3.01 * std::ldexp(1.0, -16) + (3.0 * dp + kNB) * u23 * (1.0 + 2 * u8)
+  // (the norm step adds kNB products, the last ones, at the size of both sums).
+  // Integers up to 256 are held exactly by either format.
+  const double rel = integer ? (3.0 * dp + kNB) * u23
+                     : split ? 3.01 * std::ldexp(1.0, -16) + (3.0 * dp + kNB) * u23 * (1.0 + 2 * u8)
                      : f16 ? (2 * u11 + u11 * u11) + (dp + kNB) * u23 * (1.0 + 2 * u11)
                            : (2 * u8 + u8 * u8) + (dp + kNB) * u23 * (1.0 + 2 * u8);
   const float abs_a = (f16 && !exact) ? (float)(u24 * std::sqrt((double)dp) * 1.01) : 0.0f;

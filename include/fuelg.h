@@ -64,7 +64,7 @@ extern "C" {
 #define FUELG_PREC_F16 4
 /* Let the engine pick the tier (every tier returns the same bits).  kNN /
    range / serving: d outside [32, 256] -> FP32; integer data with |v| <= 256
-   -> BF16 (its screen is exact); otherwise the fastest of the eligible
+   -> BF16 (it holds them exactly); otherwise the fastest of the eligible
    tensor-core tiers, timed on the call's first (up to) 4096 query rows the
    first time a (d, log2 n, log2 k, value class) bucket is seen, and kept for
    the process -- and in the file named by FUELG_TUNE_CACHE when that variable
