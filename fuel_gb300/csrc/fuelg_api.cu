@@ -89,6 +89,14 @@ cudaMemPool_t lib_pool() {
   return e.pool;
 }
 
+int64_t& scratch_room() {
+  thread_local int64_t room = 1ll << 62;
+  return room;
+}
+// For the tests (not in the public header): the calling thread's scratch_room, below 0
+// for no limit.
+extern "C" void fuelg_test_scratch_room(int64_t bytes) { scratch_room() = bytes < 0 ? 1ll << 62 : bytes; }
+
 CUcontext current_context() {
   using Fn = CUresult (*)(CUcontext*);
   static Fn fn = [] {

@@ -66,21 +66,35 @@ void noalloc_forget();
 void server_opened();
 void server_closed();
 
+// Bytes that the calling thread's scratch may still take: no limit, except where a
+// test of the ways out of little memory sets one (fuelg_test_scratch_room).
+int64_t& scratch_room();
+
 // Stream-ordered scratch allocations (from lib_pool) freed on scope exit.
 struct Scratch {
   void* p = nullptr;
   cudaStream_t s = nullptr;
+  int64_t taken = 0;
   Scratch() = default;
   Scratch(const Scratch&) = delete;
   Scratch& operator=(const Scratch&) = delete;
-  ~Scratch() {
-    if (p) cudaFreeAsync(p, s);
+  ~Scratch() { release(); }
+  void release() {
+    if (!p) return;
+    cudaFreeAsync(p, s);
+    p = nullptr;
+    scratch_room() += taken;
   }
   int alloc(size_t bytes, cudaStream_t stream) {
     s = stream;
     if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, lib_pool(), stream);
-    if (e != cudaSuccess) {
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if ((int64_t)bytes <= scratch_room()) e = cudaMallocFromPoolAsync(&p, bytes, lib_pool(), stream);
+    if (e == cudaSuccess) {
+      taken = (int64_t)bytes;
+      scratch_room() -= taken;
+    } else {
+      cudaGetLastError();
       p = nullptr;
       set_error("device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
       return ST_ENOMEM;
@@ -303,13 +317,13 @@ int pairwise_launch(const float* X, int64_t n, int d, int metric, int order, int
 
 // Range search, CSR output on the device.  Allocates *off/*idx/*dist with cudaMalloc.
 // radii (device, p.m entries, or nullptr): a radius per query row instead of `radius`.
-// *passes: how often every distance was formed.
+// *passes: how often every distance was formed, passes that ran out of memory included.
 int exact_range(const ExactScanParams& p, float radius, int exclude_self, int64_t** d_off, int64_t** d_idx,
                 float** d_dist, int64_t* total, int* dev_status, cudaStream_t stream, const float* radii = nullptr,
                 int* passes = nullptr);
 
 // The same in register tiles (fuelg_range.cu), d_off [p.m + 1] given: one pass, the
-// hits of a query sorted from its slots.
+// hits of a query sorted from its slots.  Adds to *passes; ST_ENOMEM leaves no result.
 bool tile_range_supported(int d);
 int tile_range(const ExactScanParams& p, float radius, int exclude_self, int64_t* d_off, int64_t** d_idx,
                float** d_dist, int64_t* total, cudaStream_t stream, const float* radii, int* passes);

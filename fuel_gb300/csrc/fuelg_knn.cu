@@ -854,9 +854,12 @@ int exact_range(const ExactScanParams& p, float radius, int exclude_self, int64_
   }
   if (p.kind == KIND_KNN && tile_range_supported(p.d)) {
     const int rc = tile_range(p, radius, exclude_self, *d_off, d_idx, d_dist, total, stream, radii, passes);
-    // (without room for the slots: the two passes below, which need none)
-    if (rc != ST_ENOMEM || *passes > 0) return rc;
-    cudaGetLastError();
+    if (rc != ST_ENOMEM) return rc;
+    // no room for the slots, or for the result beside them: the two passes below need
+    // no slots, and what the pool kept of them is handed back for the result
+    FUELG_CUDA(cudaStreamSynchronize(stream));
+    FUELG_CUDA(cudaMemPoolTrimTo(lib_pool(), 0));
+    *total = 0;
   }
   Plan pl;
   FUELG_TRY(make_plan(p, true, scan_np(p.kind, p.order), &pl));
@@ -896,7 +899,7 @@ int exact_range(const ExactScanParams& p, float radius, int exclude_self, int64_
                                                    offs, out, fill, stream);
   };
   FUELG_TRY(run(false, nullptr, nullptr));
-  *passes = 1;
+  ++*passes;
   size_t tb = 0;
   FUELG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, counts.as<int64_t>(), scanned.as<int64_t>(), mS + 1, stream));
   FUELG_TRY(tmp.alloc(tb, stream));
@@ -911,7 +914,7 @@ int exact_range(const ExactScanParams& p, float radius, int exclude_self, int64_
   FUELG_TRY(keys.alloc(sizeof(uint64_t) * tot, stream));
   FUELG_TRY(keys_sorted.alloc(sizeof(uint64_t) * tot, stream));
   FUELG_TRY(run(true, scanned.as<int64_t>(), keys.as<uint64_t>()));
-  *passes = 2;
+  ++*passes;
   size_t sb = 0;
   FUELG_CUDA(cub::DeviceSegmentedSort::SortKeys(nullptr, sb, keys.as<uint64_t>(), keys_sorted.as<uint64_t>(), tot,
                                                 p.m, *d_off, *d_off + 1, stream));

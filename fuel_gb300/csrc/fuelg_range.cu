@@ -243,6 +243,16 @@ __global__ void root_keys_kernel(uint64_t* __restrict__ keys, int64_t total) {
 
 }  // namespace
 
+// No memory for the result or the sort: nothing is left of it.
+static int no_room(int64_t** d_idx, float** d_dist, int64_t tot) {
+  if (*d_idx) cudaFree(*d_idx);
+  if (*d_dist) cudaFree(*d_dist);
+  *d_idx = nullptr;
+  *d_dist = nullptr;
+  set_error("no device memory for a range result of %lld hits", (long long)tot);
+  return ST_ENOMEM;
+}
+
 bool tile_range_supported(int d) { return d >= 1 && d <= kRangeMaxD; }
 
 int tile_range(const ExactScanParams& p, float radius, int exclude_self, int64_t* d_off, int64_t** d_idx,
@@ -283,10 +293,10 @@ int tile_range(const ExactScanParams& p, float radius, int exclude_self, int64_t
     kern<<<dim3((unsigned)qb, (unsigned)((tb + a.strip - 1) / a.strip)), 256, smem, stream>>>(a);
     ::fuelg::note_launch();
     FUELG_CUDA(cudaGetLastError());
+    ++*passes;
     return ST_OK;
   };
   FUELG_TRY(pass());
-  *passes = 1;
   size_t sb = 0;
   FUELG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, sb, counts.as<int64_t>(), d_off, p.m + 1, stream));
   FUELG_TRY(tmp.alloc(sb, stream));
@@ -297,8 +307,17 @@ int tile_range(const ExactScanParams& p, float radius, int exclude_self, int64_t
   FUELG_CUDA(cudaStreamSynchronize(stream));
   *total = tot;
   if (tot == 0) return ST_OK;
-  FUELG_CUDA(cudaMalloc(d_idx, sizeof(int64_t) * tot));
-  FUELG_CUDA(cudaMalloc(d_dist, sizeof(float) * tot));
+  Scratch keys, sorted, sort_tmp;
+  if (over) {
+    slots.release();  // the lists below take their place
+    FUELG_TRY(keys.alloc(sizeof(uint64_t) * tot, stream));
+    FUELG_TRY(sorted.alloc(sizeof(uint64_t) * tot, stream));
+  }
+  if (cudaMalloc(d_idx, sizeof(int64_t) * tot) != cudaSuccess ||
+      cudaMalloc(d_dist, sizeof(float) * tot) != cudaSuccess) {
+    cudaGetLastError();
+    return no_room(d_idx, d_dist, tot);
+  }
   if (!over) {
     range_rows_kernel<<<(unsigned)((p.m + 7) / 8), 256, 0, stream>>>(slots.as<uint64_t>(), cap, p.m, p.metric, d_off,
                                                                      *d_idx, *d_dist);
@@ -306,15 +325,11 @@ int tile_range(const ExactScanParams& p, float radius, int exclude_self, int64_t
     FUELG_CUDA(cudaGetLastError());
     return ST_OK;
   }
-  Scratch keys, sorted, sort_tmp;
-  FUELG_TRY(keys.alloc(sizeof(uint64_t) * tot, stream));
-  FUELG_TRY(sorted.alloc(sizeof(uint64_t) * tot, stream));
   FUELG_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int64_t) * p.m, stream));
   a.offs = d_off;
   a.cap = p.n;
   a.out = keys.as<uint64_t>();
   FUELG_TRY(pass());
-  *passes = 2;
   if (p.metric == METRIC_EUCLIDEAN) {
     root_keys_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, stream>>>(keys.as<uint64_t>(), tot);
     ::fuelg::note_launch();
@@ -323,7 +338,7 @@ int tile_range(const ExactScanParams& p, float radius, int exclude_self, int64_t
   sb = 0;
   FUELG_CUDA(cub::DeviceSegmentedSort::SortKeys(nullptr, sb, keys.as<uint64_t>(), sorted.as<uint64_t>(), tot, p.m,
                                                 d_off, d_off + 1, stream));
-  FUELG_TRY(sort_tmp.alloc(sb, stream));
+  if (sort_tmp.alloc(sb, stream) != ST_OK) return no_room(d_idx, d_dist, tot);
   FUELG_CUDA(cub::DeviceSegmentedSort::SortKeys(sort_tmp.p, sb, keys.as<uint64_t>(), sorted.as<uint64_t>(), tot, p.m,
                                                 d_off, d_off + 1, stream));
   return split_keys(sorted.as<uint64_t>(), tot, *d_idx, *d_dist, stream);
