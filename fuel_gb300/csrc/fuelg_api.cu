@@ -552,7 +552,8 @@ int index_topk(fuelg_index* ix, const float* Q, int64_t m, int kk, int precision
     // values outside the FP16 range (index or queries): the plain tier answers
     if (rc == ST_OK)
       rc = knn_tc_topk(ix->tc, Q, m, ix->X, kk, ix->order, ix->metric, tier, keys, dstat, s, rescored, &exact);
-    if (rc != ST_OK && rc != ST_ENOTSUP) return rc;
+    // (nor without room for its lists)
+    if (rc != ST_OK && rc != ST_ENOTSUP && rc != ST_ENOMEM) return rc;
     if (rc == ST_OK) {
       // integers that screen exactly take the one-product form whatever the split request
       *used = tier == TC_F16 ? FUELG_PREC_F16 : (tier == TC_SPLIT && !exact) ? FUELG_PREC_SPLIT_BF16 : FUELG_PREC_BF16;
@@ -1196,8 +1197,14 @@ int fuelg_knn_f64(fuelg_index* ix, const double* queries, int64_t m, int32_t k, 
     FUELG_TRY(f64_screen_build(ix->X64, ix->n, ix->d, s, &ix->screen));
     ix->screen_tried = true;
   }
-  FUELG_TRY(f64_knn(f64_view(ix), Q, m, k, exclude_mode, static_cast<int64_t*>(oi.dptr),
-                    static_cast<double*>(od.dptr), s));
+  F64Scan view = f64_view(ix);
+  int rc = f64_knn(view, Q, m, k, exclude_mode, static_cast<int64_t*>(oi.dptr), static_cast<double*>(od.dptr), s);
+  if (rc == ST_ENOMEM && view.screen != nullptr) {
+    // no room for the screen's lists: the FP64 scan, whose batches fit
+    view.screen = nullptr;
+    rc = f64_knn(view, Q, m, k, exclude_mode, static_cast<int64_t*>(oi.dptr), static_cast<double*>(od.dptr), s);
+  }
+  FUELG_TRY(rc);
   int64_t d2h = 0;
   FUELG_TRY(oi.flush(s, &d2h));
   FUELG_TRY(od.flush(s, &d2h));

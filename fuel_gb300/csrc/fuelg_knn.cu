@@ -373,8 +373,10 @@ int exact_topk(const ExactScanParams& p, uint64_t* out_keys, int* dev_status, cu
   // 326 in tiles at n = 100, 382 and 434 at n = 500; 200 000 queries, k = 20,
   // d = 2, n = 1000 take 1796 and 1163; 2000 queries, k = 10, d = 16, n = 2000
   // take 170 and 111.
-  if (p.kind == KIND_KNN && p.n >= kTileMinRows && tile_scan_supported(p.d, p.kk))
-    return tile_scan_topk(p, out_keys, dev_status, stream);
+  if (p.kind == KIND_KNN && p.n >= kTileMinRows && tile_scan_supported(p.d, p.kk)) {
+    const int rc = tile_scan_topk(p, out_keys, dev_status, stream);
+    if (rc != ST_ENOMEM) return rc;  // (without room for its lists: the scan below, whose are smaller)
+  }
   const bool kk1 = p.kk == 1;
   Plan pl;
   FUELG_TRY(make_plan(p, kk1, scan_np(p.kind, p.order), &pl));

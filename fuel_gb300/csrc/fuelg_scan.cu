@@ -316,9 +316,10 @@ int tile_scan_topk(const ExactScanParams& p, uint64_t* out_keys, int* dev_status
   // than the others holds them up less often (20 000-point self-join, d = 16: 1.24
   // ms with 1, 1.15 with 2, 1.09 with 4, 1.34 with 6, where one CTA per SM is left)
   const int tps = p.d <= 16 ? 4 : p.d <= 32 ? 2 : 1;
-  // queries in batches whose run lists stay below 1 GiB
-  const int64_t mb_max =
-      std::max<int64_t>(64, (int64_t)((1ull << 30) / ((size_t)p.kk * 8 * 2)) / 64 * 64);
+  // queries in batches whose lists stay below 1 GiB: those of the runs, or (kk > 32,
+  // a block per CTA) the kept keys with their logs
+  const size_t qwords = std::max<size_t>(2 * (size_t)p.kk, small ? 0 : lstride);
+  const int64_t mb_max = std::max<int64_t>(64, (int64_t)((1ull << 30) / (8 * qwords)) / 64 * 64);
   for (int64_t b0 = 0; b0 < p.m; b0 += mb_max) {
     const int64_t m = std::min<int64_t>(mb_max, p.m - b0);
     // few queries: fewer warps per CTA, so that no warp holds only padding rows

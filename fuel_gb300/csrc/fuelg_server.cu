@@ -118,7 +118,8 @@ int run_batch(fuelg_server* sv, std::vector<Request*>& batch, cudaStream_t s, fl
     int exact = 0;
     rc = knn_tc_topk(ix.tc, q.as<float>(), m, ix.X, kmax, ix.order, ix.metric, tier, keys.as<uint64_t>(),
                      dstat.as<int>(), s, &rescored, &exact, rk.as<int32_t>());
-    if (rc != ST_OK && rc != ST_ENOTSUP) return rc;  // ENOTSUP: queries outside the FP16 range
+    // ENOTSUP: queries outside the FP16 range; ENOMEM: no room for the screen's lists
+    if (rc != ST_OK && rc != ST_ENOTSUP && rc != ST_ENOMEM) return rc;
   }
   if (rc != ST_OK) {
     ExactScanParams p;
