@@ -619,9 +619,10 @@ int resolve_knn_precision(fuelg_index* ix, const float* Q, int64_t m, int kk, in
   *out = FUELG_PREC_FP32;
   if (ix->n == 0 || !knn_tc_supported(ix->n, ix->d, kk, TC_BF16)) return ST_OK;
   if (!ix->tc) FUELG_TRY(knn_tc_index_build(ix->X, ix->n, ix->d, s, &ix->tc));
+  if (!knn_tc_index_screens(ix->tc)) return ST_OK;  // no tier runs: nothing to time or to record
   const int cls = knn_tc_index_class(ix->tc);
   if (cls == TC_CLASS_INTEGER) {
-    *out = FUELG_PREC_BF16;  // exact screen, no margin, no re-score
+    *out = FUELG_PREC_BF16;  // exact operands: one product, no re-score where the screen is exact
     return ST_OK;
   }
   const TuneKey key{ix->d, ilog2_floor(ix->n), ilog2_floor(2 * (int64_t)kk - 1), cls};
@@ -643,7 +644,7 @@ int resolve_knn_precision(fuelg_index* ix, const float* Q, int64_t m, int kk, in
   const int cand_wide[2] = {FUELG_PREC_SPLIT_BF16, FUELG_PREC_BF16};
   const int* cand = cls == TC_CLASS_F16_RANGE ? cand_f16 : cand_wide;
   const int nc = cls == TC_CLASS_F16_RANGE ? 3 : 2;
-  int best = FUELG_PREC_SPLIT_BF16;
+  int best = FUELG_PREC_FP32;
   float best_ms = 1e30f;
   for (int c = 0; c < nc; c++) {
     int used = 0;
@@ -657,9 +658,10 @@ int resolve_knn_precision(fuelg_index* ix, const float* Q, int64_t m, int kk, in
       best = cand[c];
     }
   }
+  *out = best;
+  if (best == FUELG_PREC_FP32) return ST_OK;  // none ran (this call's values or memory): not the bucket's answer
   std::lock_guard<std::mutex> lk(g_tune_mu);
   tune_store_locked(key, best);
-  *out = best;
   return ST_OK;
 }
 

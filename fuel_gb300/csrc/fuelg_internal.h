@@ -281,6 +281,8 @@ void knn_tc_index_free(TcIndex* t);
 // sums cannot round), values within the FP16 range, or wider values.
 constexpr int TC_CLASS_INTEGER = 0, TC_CLASS_F16_RANGE = 1, TC_CLASS_WIDE = 2;
 int knn_tc_index_class(const TcIndex* t);
+// Whether the index's norms leave room for a screen (knn_tc_topk: ST_ENOTSUP otherwise).
+bool knn_tc_index_screens(const TcIndex* t);
 int knn_tc_index_add_lo(TcIndex* t, const float* X32, cudaStream_t stream);
 // FP16 copy of the index; ST_ENOTSUP when a value lies outside the FP16 range.
 int knn_tc_index_add_f16(TcIndex* t, const float* X32, cudaStream_t stream);

@@ -1328,6 +1328,8 @@ int knn_tc_index_class(const TcIndex* t) {
   return t->vmax <= kF16Max ? TC_CLASS_F16_RANGE : TC_CLASS_WIDE;
 }
 
+bool knn_tc_index_screens(const TcIndex* t) { return t->xmax_n2 < 1e37f; }
+
 void knn_tc_index_free(TcIndex* t) {
   if (!t) return;
   if (t->xb) cudaFree(t->xb);
@@ -1420,7 +1422,7 @@ int knn_tc_topk(const TcIndex* ti, const float* Q32, int64_t m, const float* X32
   const int64_t n = ti->n;
   const int d = ti->d;
   const int dp = ti->dp;
-  if (!(ti->xmax_n2 < 1e37f)) {
+  if (!knn_tc_index_screens(ti)) {
     // norms near or past the FP32 range have no useful screen: the exact scan answers
     set_error("index norms exceed the tensor-core screen's range (max |x|^2 = %g)", (double)ti->xmax_n2);
     return ST_ENOTSUP;
