@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
   const int64_t G = gridDim.x;
   const int64_t t_end = scan_run_begin(blockIdx.x + 1, a.T, G);
   uint64_t* const my = a.lists + ((size_t)blockIdx.x * QM + warp * kTileQ) * a.lstride;  // this warp's rows
-  int polled = 0, stop = 0;
+  int stop = 0;  // thread 0: the cancel word as of its last look
 
   // lane 0: row r's new limit from its kk-th key (never above what other runs of
   // the query have found).  gthr has m words: rows past m, which keep index rows of
@@ -126,16 +126,16 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
     int buf = 0;
     bool stopped = false;
     for (int64_t x0 = x_first; x0 < x_last; x0 += a.tps, buf ^= 1) {
-      if (threadIdx.x == 0 && a.cancel != nullptr && (++polled & 15) == 0 && *a.cancel) {
-        stop = 1;
-        atomicOr(a.status, DEV_CANCELLED);
-      }
       cp_async_wait_all();
       // these tiles have landed; the other buffer is no longer read
       if (__syncthreads_or(stop)) {
+        if (threadIdx.x == 0) atomicOr(a.status, DEV_CANCELLED);
         stopped = true;
         break;
       }
+      // a look every 16 tiles, from the index's first ones on (an index of few tiles has no
+      // 16th stage), whose answer the next barrier takes: none waits for host memory
+      if (threadIdx.x == 0 && a.cancel != nullptr && ((int)x0 & 15) < a.tps) stop = *a.cancel;
       // the other runs' limits as of this stage (used from the next one on)
       unsigned seen = 0xffffffffu;
       if (a.gthr != nullptr && lane < kTileQ && q0 + warp * kTileQ + lane < a.m)
