@@ -312,14 +312,17 @@ __global__ void __launch_bounds__(kT) narrow64_kernel(const double* __restrict__
     for (int c = lane; c < d; c += 32) {
       const double x = X[r * d + c], c0 = isfinite(centre[c]) ? centre[c] : 0.0;
       const double v = __dsub_rn(x, c0);
-      // what the subtraction rounded away (the two-sum of x and -c0; NaN past the range)
-      const double t = __dsub_rn(v, x);
-      const double lost = __dsub_rn(__dsub_rn(x, __dsub_rn(v, t)), __dadd_rn(c0, t));
       const float f = __double2float_rn(v);
       out[r * d + c] = f;
       const double e = fabs(v - (double)f) + 1.2e-16 * fabs(v);  // and the shift's own rounding
       e2 = fma(e, e, e2);
-      vm = f == rintf(f) && v == (double)f && lost == 0.0 ? fmaxf(vm, fabsf(f)) : __int_as_float(0x7f800000);
+      float iv = __int_as_float(0x7f800000);
+      if (f == rintf(f) && v == (double)f) {  // (FP64 is slow here: few values of other data come this far)
+        // what the subtraction rounded away: the two-sum of x and -c0
+        const double t = __dsub_rn(v, x);
+        if (__dsub_rn(__dsub_rn(x, __dsub_rn(v, t)), __dadd_rn(c0, t)) == 0.0) iv = fabsf(f);
+      }
+      vm = fmaxf(vm, iv);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
