@@ -211,9 +211,11 @@ __device__ __forceinline__ f32x2 exact_dist_pair(const f32x2 (&x)[D], const f32x
 }
 
 // One iteration over all problems: assignment + sum updates of changed points.
-// Problems of 2 or 8 dimensions whose centres fit (every such problem up to 2048
-// centres): two centres per packed step, their coordinates interleaved in shared
-// memory.  WIDE: some problem has 32 or 64 dimensions, whose rows are held in
+// Problems of 2 or 8 dimensions (two of the four widths whose rows are held in
+// registers; others take fuel's order from memory) whose centres fit the stage, up to
+// 8192 and 2048: two centres per packed step, their coordinates interleaved in shared
+// memory; with more centres one at a time, from global memory (10 passes of 100 000 x 2,
+// k = 8200 9.1 ms, 200 000 x 8, k = 2100 9.7; 29.5 and 35.7 through the general loop).  WIDE: some problem has 32 or 64 dimensions, whose rows are held in
 // registers (128 per thread; 64 without).  Bound by FP32 issue and, in the first
 // passes, by the adds of changed rows: a later pass over 10.3 million rows of 2 or
 // 8 dimensions, k to 256: 0.90 -> 0.56 ms against one centre at a time.
@@ -346,6 +348,8 @@ __global__ void __launch_bounds__(kItemRows) batched_assign_kernel(
       else if (paired) scan_pairs(Dim<8>{});
       else if (WIDE && pr.d == 32) scan(Dim<32>{});
       else if (WIDE && pr.d == 64) scan(Dim<64>{});
+      else if (pr.d == 2) scan(Dim<2>{});  // (centres that are not staged)
+      else if (pr.d == 8) scan(Dim<8>{});
       else {
           for (int c = 0; c < pr.k; c++) {
             const float dv = exact_dist_scalar<KIND, ORDER>(xr, C + pr.c_off + (int64_t)c * pr.d, pr.d);
