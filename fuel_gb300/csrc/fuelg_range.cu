@@ -25,7 +25,7 @@ constexpr int kRangeMaxD = 128;
 constexpr int kMaxStrip = 8;                // most 128-row tiles that one CTA works through
 constexpr int kTwoPerSm = 2 * 152;          // places on the chip with two CTAs per SM
 constexpr int kTwoCtas = 112 * 1024;        // shared memory with which two CTAs fit an SM
-// Most slots of a query: what a block sorts in the shared memory that lets five
+// Most slots of a query: what a block sorts in the shared memory that lets six
 // blocks share an SM.  (With 1024 the 300-hit self-join had rows past them and took
 // 4.29 ms for 1.74.)
 constexpr int kSlots = 4096;
@@ -41,7 +41,9 @@ struct RangeTileArgs {
   float radius;
   const float* radii;  // [m] or nullptr
   int exclude_self;
-  unsigned long long* counts;  // [m] hits so far; then [m]: a zero, [m + 1]: set when a query has more than cap
+  // [m] hits so far; then [m]: a zero, [m + 1]: set when a query has more than cap, [m + 2]:
+  // more than kWarpSort
+  unsigned long long* counts;
   const int64_t* offs;         // [m] where a query's keys start, or nullptr: at query * cap
   int64_t cap;                 // most keys written for a query
   uint64_t* out;               // keys (squared distance, index)
@@ -127,6 +129,7 @@ __global__ void __launch_bounds__(256, 2) range_tile_kernel(RangeTileArgs a) {
       if (cnt > 0) {
         const int64_t q = qw + lane;
         const int64_t base = (int64_t)atomicAdd(a.counts + q, (unsigned long long)cnt);
+        if (base + cnt > kWarpSort) a.counts[a.m + 2] = 1;
         if (base + cnt > a.cap) a.counts[a.m + 1] = 1;
         else place = a.out + (a.offs != nullptr ? a.offs[q] : q * a.cap) + base;
       }
@@ -176,62 +179,104 @@ __device__ __forceinline__ void warp_sort_slots(const uint64_t* __restrict__ in,
   else sort_slots<8>(in, c, metric, lane, put);
 }
 
-// A query's slots sorted into its place of the result: a warp per query, in
-// registers.  A query with more than kWarpSort keys by the whole block: pieces of up
-// to kWarpSort keys, sorted by a warp each, and every key's rank from its place
-// in its own piece and a binary search in each of the others.  0.33 ms for the same
-// self-join (a segmented sort over all lists and a split of its keys: 1.25).
-// Whole calls: that one 4.32 -> 1.74 ms, 20 000 x 20 000 x 16 with 19 hits a row
-// 2.83 -> 1.23, 40 queries on 40 000 x 64 0.92 -> 0.13; with 3900 hits a row, many
-// lists past the slots, 11.8 -> 11.7.
+// A query's slots sorted into its place of the result, up to kWarpSort keys: a warp
+// per query, in registers.
 __global__ void __launch_bounds__(256) range_rows_kernel(const uint64_t* __restrict__ slots, int64_t cap, int64_t m,
                                                          int metric, const int64_t* __restrict__ offs,
                                                          int64_t* __restrict__ idx, float* __restrict__ dist) {
-  __shared__ uint64_t s_key[kSlots];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t q0 = (int64_t)blockIdx.x * 8;
-  const int64_t q = q0 + warp;
-  int c = 0;
-  if (q < m) {
-    const int64_t o = offs[q];
-    c = (int)(offs[q + 1] - o);
-    if (c > 0 && c <= kWarpSort)
-      warp_sort_slots(slots + q * cap, c, metric, lane, [&](int e, uint64_t key) {
-        idx[o + e] = key_idx(key);
-        dist[o + e] = key_dist(key);
-      });
+  const int64_t q = (int64_t)blockIdx.x * 8 + warp;
+  if (q >= m) return;
+  const int64_t o = offs[q], c = offs[q + 1] - o;
+  if (c > 0 && c <= kWarpSort)
+    warp_sort_slots(slots + q * cap, (int)c, metric, lane, [&](int e, uint64_t key) {
+      idx[o + e] = key_idx(key);
+      dist[o + e] = key_dist(key);
+    });
+}
+
+// The longer lists, up to kSlots keys, a block each (other queries' blocks leave at
+// once), by merging: a thread sorts V keys in registers, then runs are merged two by
+// two, a thread making V consecutive keys of every merge from where their ranks split
+// the two runs (the merge path of Green, McColl and Bader).  A key costs some 30
+// instructions in the registers' network and 20 a merge; a warp's network of 256 costs
+// 300.  Keys sit one past every 16 in shared memory, so that a warp's threads, V keys
+// apart, use different banks.  27 lists of 3365 keys 27 us, 2211 of 2344 137; eight lists
+// to a block, one after the other by ranks among sorted pieces, and whole calls: 849 us
+// (now 115; the two-pass scan with a segmented sort 227) and 760 (398; 484).
+__device__ __forceinline__ int list_pos(int e) { return e + (e >> 4); }
+
+template <int V>
+__device__ __forceinline__ void sort_list(const uint64_t* __restrict__ in, int n, int metric, uint64_t* s_key) {
+  uint64_t v[V];
+#pragma unroll
+  for (int r = 0; r < V; r++) {
+    const int e = (int)threadIdx.x + 256 * r;
+    v[r] = e < n ? range_key(in[e], metric) : KEY_NONE;
   }
-  if (!__syncthreads_or(c > kWarpSort)) return;
-  for (int w = 0; w < 8 && q0 + w < m; w++) {
-    const int64_t o = offs[q0 + w];
-    const int n = (int)(offs[q0 + w + 1] - o);
-    if (n <= kWarpSort) continue;
-    const uint64_t* in = slots + (q0 + w) * cap;
-    const int pieces = (n + kWarpSort - 1) / kWarpSort, len = (n + pieces - 1) / pieces;
-    __syncthreads();  // the previous query's keys are no longer read
-    for (int p = warp; p < pieces; p += 8) {
-      const int b = p * len;
-      warp_sort_slots(in + b, min(len, n - b), metric, lane, [&](int e, uint64_t key) { s_key[b + e] = key; });
+#pragma unroll
+  for (int k2 = 2; k2 <= V; k2 <<= 1)
+#pragma unroll
+    for (int j = k2 >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int r = 0; r < V; r++) {
+        if (r & j) continue;
+        const uint64_t x = v[r], y = v[r ^ j];
+        const bool sw = (r & k2) == 0 ? x > y : x < y;
+        v[r] = sw ? y : x;
+        v[r ^ j] = sw ? x : y;
+      }
+  const int k0 = (int)threadIdx.x * V;  // this thread's keys of every merge: [k0, k0 + V)
+#pragma unroll
+  for (int r = 0; r < V; r++) s_key[list_pos(k0 + r)] = v[r];
+  __syncthreads();
+#pragma unroll 1
+  for (int w = V; w < 256 * V; w *= 2) {
+    const int a = k0 & ~(2 * w - 1), b = a + w, k = k0 - a;  // runs at a and b; k keys of the merge come before
+    int lo = max(0, k - w), hi = min(k, w);  // how many of those are of the first run
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (s_key[list_pos(a + mid)] < s_key[list_pos(b + k - 1 - mid)]) lo = mid + 1;
+      else hi = mid;
+    }
+    int i = lo, j = k - lo;
+    uint64_t va = i < w ? s_key[list_pos(a + i)] : KEY_NONE, vb = j < w ? s_key[list_pos(b + j)] : KEY_NONE;
+#pragma unroll
+    for (int r = 0; r < V; r++) {
+      const bool first = j >= w || (i < w && va <= vb);
+      v[r] = first ? va : vb;
+      if (first) i++;
+      else j++;
+      const uint64_t next = first ? (i < w ? s_key[list_pos(a + i)] : KEY_NONE)
+                                  : (j < w ? s_key[list_pos(b + j)] : KEY_NONE);
+      va = first ? next : va;
+      vb = first ? vb : next;
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < n; e += 256) {
-      const uint64_t key = s_key[e];
-      const int own = e / len;
-      int rank = e - own * len;
-      for (int p = 0; p < pieces; p++) {
-        if (p == own) continue;
-        const uint64_t* s = s_key + p * len;
-        int lo = 0, hi = min(len, n - p * len);  // keys below: [0, lo) are, [hi, ..) are not
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (s[mid] < key) lo = mid + 1;
-          else hi = mid;
-        }
-        rank += lo;
-      }
-      idx[o + rank] = key_idx(key);
-      dist[o + rank] = key_dist(key);
-    }
+#pragma unroll
+    for (int r = 0; r < V; r++) s_key[list_pos(k0 + r)] = v[r];
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(256) range_long_kernel(const uint64_t* __restrict__ slots, int64_t cap, int metric,
+                                                         const int64_t* __restrict__ offs, int64_t* __restrict__ idx,
+                                                         float* __restrict__ dist) {
+  static_assert(kSlots == 256 * 16 && kWarpSort == 256, "2 to 16 keys per thread");
+  __shared__ uint64_t s_key[kSlots + kSlots / 16];
+  const int64_t q = blockIdx.x;
+  const int64_t o = offs[q];
+  if (offs[q + 1] - o <= kWarpSort) return;
+  const int n = (int)(offs[q + 1] - o);
+  const uint64_t* in = slots + q * cap;
+  if (n <= 512) sort_list<2>(in, n, metric, s_key);
+  else if (n <= 1024) sort_list<4>(in, n, metric, s_key);
+  else if (n <= 2048) sort_list<8>(in, n, metric, s_key);
+  else sort_list<16>(in, n, metric, s_key);
+  for (int e = threadIdx.x; e < n; e += 256) {
+    const uint64_t key = s_key[list_pos(e)];
+    idx[o + e] = key_idx(key);
+    dist[o + e] = key_dist(key);
   }
 }
 
@@ -243,10 +288,13 @@ __global__ void root_keys_kernel(uint64_t* __restrict__ keys, int64_t total) {
 
 }  // namespace
 
-// No memory for the result or the sort: nothing is left of it.
-static int no_room(int64_t** d_idx, float** d_dist, int64_t tot) {
-  if (*d_idx) cudaFree(*d_idx);
-  if (*d_dist) cudaFree(*d_dist);
+// The result's arrays, both or neither.
+static int result_alloc(int64_t** d_idx, float** d_dist, int64_t tot) {
+  if (cudaMalloc(d_idx, sizeof(int64_t) * tot) == cudaSuccess) {
+    if (cudaMalloc(d_dist, sizeof(float) * tot) == cudaSuccess) return ST_OK;
+    cudaFree(*d_idx);
+  }
+  cudaGetLastError();
   *d_idx = nullptr;
   *d_dist = nullptr;
   set_error("no device memory for a range result of %lld hits", (long long)tot);
@@ -258,8 +306,8 @@ bool tile_range_supported(int d) { return d >= 1 && d <= kRangeMaxD; }
 int tile_range(const ExactScanParams& p, float radius, int exclude_self, int64_t* d_off, int64_t** d_idx,
                float** d_dist, int64_t* total, cudaStream_t stream, const float* radii, int* passes) {
   Scratch counts, tmp, slots;
-  FUELG_TRY(counts.alloc(sizeof(int64_t) * (p.m + 2), stream));
-  FUELG_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int64_t) * (p.m + 2), stream));
+  FUELG_TRY(counts.alloc(sizeof(int64_t) * (p.m + 3), stream));
+  FUELG_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int64_t) * (p.m + 3), stream));
   const int64_t cap = std::min<int64_t>(
       p.n, std::clamp<int64_t>((int64_t)(kSlotBytes / sizeof(uint64_t)) / p.m, 32, kSlots));
   FUELG_TRY(slots.alloc(sizeof(uint64_t) * cap * p.m, stream));
@@ -301,30 +349,29 @@ int tile_range(const ExactScanParams& p, float radius, int exclude_self, int64_t
   FUELG_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, sb, counts.as<int64_t>(), d_off, p.m + 1, stream));
   FUELG_TRY(tmp.alloc(sb, stream));
   FUELG_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, sb, counts.as<int64_t>(), d_off, p.m + 1, stream));
-  int64_t tot = 0, over = 0;
+  int64_t tot = 0, flags[2] = {0, 0};
   FUELG_CUDA(cudaMemcpyAsync(&tot, d_off + p.m, sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
-  FUELG_CUDA(cudaMemcpyAsync(&over, counts.as<int64_t>() + p.m + 1, sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
+  FUELG_CUDA(cudaMemcpyAsync(flags, counts.as<int64_t>() + p.m + 1, sizeof(flags), cudaMemcpyDeviceToHost, stream));
   FUELG_CUDA(cudaStreamSynchronize(stream));
+  const bool over = flags[0] != 0, longer = flags[1] != 0;
   *total = tot;
   if (tot == 0) return ST_OK;
-  Scratch keys, sorted, sort_tmp;
-  if (over) {
-    slots.release();  // the lists below take their place
-    FUELG_TRY(keys.alloc(sizeof(uint64_t) * tot, stream));
-    FUELG_TRY(sorted.alloc(sizeof(uint64_t) * tot, stream));
-  }
-  if (cudaMalloc(d_idx, sizeof(int64_t) * tot) != cudaSuccess ||
-      cudaMalloc(d_dist, sizeof(float) * tot) != cudaSuccess) {
-    cudaGetLastError();
-    return no_room(d_idx, d_dist, tot);
-  }
   if (!over) {
+    FUELG_TRY(result_alloc(d_idx, d_dist, tot));
     range_rows_kernel<<<(unsigned)((p.m + 7) / 8), 256, 0, stream>>>(slots.as<uint64_t>(), cap, p.m, p.metric, d_off,
                                                                      *d_idx, *d_dist);
     ::fuelg::note_launch();
+    if (longer) {
+      range_long_kernel<<<(unsigned)p.m, 256, 0, stream>>>(slots.as<uint64_t>(), cap, p.metric, d_off, *d_idx, *d_dist);
+      ::fuelg::note_launch();
+    }
     FUELG_CUDA(cudaGetLastError());
     return ST_OK;
   }
+  slots.release();  // the lists take their place
+  Scratch keys, sorted, sort_tmp;
+  FUELG_TRY(keys.alloc(sizeof(uint64_t) * tot, stream));
+  FUELG_TRY(sorted.alloc(sizeof(uint64_t) * tot, stream));
   FUELG_CUDA(cudaMemsetAsync(counts.p, 0, sizeof(int64_t) * p.m, stream));
   a.offs = d_off;
   a.cap = p.n;
@@ -338,9 +385,10 @@ int tile_range(const ExactScanParams& p, float radius, int exclude_self, int64_t
   sb = 0;
   FUELG_CUDA(cub::DeviceSegmentedSort::SortKeys(nullptr, sb, keys.as<uint64_t>(), sorted.as<uint64_t>(), tot, p.m,
                                                 d_off, d_off + 1, stream));
-  if (sort_tmp.alloc(sb, stream) != ST_OK) return no_room(d_idx, d_dist, tot);
+  FUELG_TRY(sort_tmp.alloc(sb, stream));
   FUELG_CUDA(cub::DeviceSegmentedSort::SortKeys(sort_tmp.p, sb, keys.as<uint64_t>(), sorted.as<uint64_t>(), tot, p.m,
                                                 d_off, d_off + 1, stream));
+  FUELG_TRY(result_alloc(d_idx, d_dist, tot));  // (120 us or more of host time, beside the sort)
   return split_keys(sorted.as<uint64_t>(), tot, *d_idx, *d_dist, stream);
 }
 
