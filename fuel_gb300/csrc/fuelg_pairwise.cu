@@ -14,10 +14,11 @@
 // form is the same value.
 //
 // Kernels: d <= 128 (pairwise_tile_kernel): blocks of 64 rows against strips of
-// 128-column tiles in the register tiles of fuelg_tile.cuh.  Larger d
-// (pairwise_kernel): 32 x 32 tiles of the lower tile triangle, 64-column chunks,
-// 2 x 2 pairs with 8 lane accumulators each.  Small d is bound by FP32 issue and
-// the output writes (HBM), large d by FP32 issue.
+// 128-column tiles in the register tiles of fuelg_tile.cuh; where those would leave
+// places on the chip empty (pairwise_rows_kernel), 64 x 64 tiles with half the pairs per
+// thread.  Larger d (pairwise_kernel): 32 x 32 tiles of the lower tile triangle,
+// 64-column chunks, 2 x 2 pairs with 8 lane accumulators each.  Small d is bound by FP32
+// issue and the output writes (HBM), large d by FP32 issue, few rows by latency.
 #include <algorithm>
 #include <cmath>
 
@@ -143,6 +144,104 @@ __global__ void __launch_bounds__(256) pairwise_kernel(const float* __restrict__
   }
 }
 
+// Few rows: 64 x 64 tiles of the lower tile triangle, whole rows of both blocks in
+// shared memory, 4 x 4 pairs per thread computed lane by lane -- lane l's sum over the
+// 8-blocks is finished before it is added to the running total, which is the
+// reference's order (acc_0 + acc_1 + ... + acc_7, then the tail) with 2 registers per pair
+// instead of 9.  Half the serial work per thread of the tiles below, which is what a
+// call takes that does not fill the chip (pairwise_launch: both sides measured).
+constexpr int PR = 64;
+template <int ORDER, int METRIC, int FORM>
+__global__ void __launch_bounds__(256) pairwise_rows_kernel(const float* __restrict__ X, int64_t n, int d,
+                                                            int64_t ntb, float* __restrict__ out) {
+  constexpr bool FMA8 = ORDER == ORDER_X86;
+  extern __shared__ float rs[];  // [2][PR][d + 1]: row block i, row block j
+  __shared__ float st[PR][PR + 1];
+  const int S = d + 1;  // odd stride: the 16 rows a half-warp reads sit in different banks
+  float* sa = rs;
+  float* sb = rs + PR * S;
+  const int64_t t = blockIdx.x;
+  int64_t bi = (int64_t)((std::sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
+  while (bi * (bi + 1) / 2 > t) bi--;
+  while ((bi + 1) * (bi + 2) / 2 <= t) bi++;
+  const int64_t bj = t - bi * (bi + 1) / 2;
+  if (bi >= ntb) return;
+  const int64_t i0 = bi * PR, j0 = bj * PR;
+  for (int e = threadIdx.x; e < PR * d; e += 256) {
+    const int r = e / d, c = e - r * d;
+    const int64_t gi = i0 + r, gj = j0 + r;
+    sa[r * S + c] = gi < n ? __ldg(X + gi * d + c) : 0.0f;
+    sb[r * S + c] = gj < n ? __ldg(X + gj * d + c) : 0.0f;
+  }
+  __syncthreads();
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // rows ty + 16a, cols tx + 16b
+  const int sd = d & ~7;
+  float sum[4][4];
+#pragma unroll 1
+  for (int l = 0; l < 8; l++) {
+    float acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) acc[a][b] = 0.0f;
+    for (int c = l; c < sd; c += 8) {
+      float xa[4], yb[4];
+#pragma unroll
+      for (int a = 0; a < 4; a++) xa[a] = sa[(ty + 16 * a) * S + c];
+#pragma unroll
+      for (int b = 0; b < 4; b++) yb[b] = sb[(tx + 16 * b) * S + c];
+#pragma unroll
+      for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+          const float df = __fsub_rn(xa[a], yb[b]);
+          acc[a][b] = FMA8 ? __fmaf_rn(df, df, acc[a][b]) : __fadd_rn(sq_rn(df), acc[a][b]);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) sum[a][b] = l == 0 ? acc[a][b] : __fadd_rn(sum[a][b], acc[a][b]);
+  }
+  for (int c = sd; c < d; c++) {
+    float xa[4], yb[4];
+#pragma unroll
+    for (int a = 0; a < 4; a++) xa[a] = sa[(ty + 16 * a) * S + c];
+#pragma unroll
+    for (int b = 0; b < 4; b++) yb[b] = sb[(tx + 16 * b) * S + c];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) {
+        const float df = __fsub_rn(xa[a], yb[b]);
+        sum[a][b] = FMA8 ? __fmaf_rn(df, df, sum[a][b]) : __fadd_rn(sum[a][b], sq_rn(df));
+      }
+  }
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    const int64_t gi = i0 + ty + 16 * a;
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const int64_t gj = j0 + tx + 16 * b;
+      const float v = METRIC == METRIC_EUCLIDEAN ? __fsqrt_rn(sum[a][b]) : sum[a][b];
+      if (FORM == FUELG_PAIRWISE_CONDENSED) {
+        if (gi < n && gj < gi) out[gi * (gi - 1) / 2 + gj] = v;
+      } else {
+        if (gi < n && gj < n) out[gi * n + gj] = v;
+        st[ty + 16 * a][tx + 16 * b] = v;
+      }
+    }
+  }
+  if (FORM == FUELG_PAIRWISE_SQUARE && bi != bj) {  // the mirrored tile (j, i), row by row
+    __syncthreads();
+    for (int e = threadIdx.x; e < PR * PR; e += 256) {
+      const int rj = e / PR, ci = e - rj * PR;
+      const int64_t gj = j0 + rj, gi = i0 + ci;
+      if (gj < n && gi < n) out[gj * n + gi] = st[ci][rj];
+    }
+  }
+}
+
 constexpr int kRows = kTileQ * kTileMaxWarps;  // 64 rows of a block
 constexpr int kTileMaxD = 128;
 constexpr int kMaxStrip = 8;                    // most 128-column tiles that one CTA works through
@@ -159,7 +258,7 @@ constexpr int kMirror = kTileP * (kRows + 1);   // floats of the square form's t
 // lane steps, 119 us of writes).  Whole calls against 64 x 64 tiles with 4 x 4
 // pairs per thread, condensed: 20000 x 16 722 -> 413 us (Euclidean 798 -> 494),
 // 20000 x 3 382 -> 206, 20000 x 128 3482 -> 2942; square 20000 x 16 873 -> 649,
-// 5000 x 64 175 -> 144; up to 1000 rows equal (34, launch and copy).
+// 5000 x 64 175 -> 144.
 template <bool FMA8, int METRIC, int FORM, int BUFS>
 __global__ void __launch_bounds__(256, 2) pairwise_tile_kernel(const float* __restrict__ X, int64_t n, int d, int nb,
                                                                int strip, f32x2 nz, float* __restrict__ out) {
@@ -241,8 +340,8 @@ int pairwise_launch(const float* X, int64_t n, int d, int metric, int order, int
                     cudaStream_t stream) {
   if (n < 2 && form == FUELG_PAIRWISE_CONDENSED) return ST_OK;
   if (n < 1) return ST_OK;
-  const bool tile = d <= kTileMaxD;
-  const int64_t ntb = (n + PT - 1) / PT;
+  const bool wide = d > kTileMaxD;
+  const int64_t ntb = (n + (wide ? PT : PR) - 1) / (wide ? PT : PR);
   const int64_t tiles = ntb * (ntb + 1) / 2;
   if (tiles > 0x7fffffffll) {
     set_error("pairwise: %lld points need more tiles than one launch holds", (long long)n);
@@ -261,8 +360,17 @@ int pairwise_launch(const float* X, int64_t n, int d, int metric, int order, int
   // place on the chip: strips of eight at any n took 253 us at 5000 x 64 (144), 54
   // at 1000 x 16 (34)
   const int strip = (int)std::clamp<int64_t>(rb * cb / 2 / (kTwoPerSm * 4), 1, kMaxStrip);
-  auto launch = [&](auto k1, auto k2, auto kc) -> int {
-    if (tile) {
+  // 64 x 64 tiles while all of them are resident at once, up to 1536 rows.  Kernel, us, 64 x
+  // 64 / 64 x 128: n = 300, d = 64 13.8 / 17.9, d = 128 19.8 / 28.5; n = 1500, d = 8 10.1 / 10.0,
+  // d = 64 20.0 / 26.0, d = 128 30.1 / 43.2; n = 1700, d = 8 12.3 / 10.3, d = 64 25.9 / 25.9,
+  // n = 1900, d = 128 52.8 / 43.2.
+  const bool few = tiles <= kTwoPerSm;
+  auto launch = [&](auto kr, auto k1, auto k2, auto kc) -> int {
+    if (!wide && few) {
+      const size_t rsm = sizeof(float) * 2 * PR * (d + 1);
+      FUELG_CUDA(cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rsm));
+      kr<<<(unsigned)tiles, 256, rsm, stream>>>(X, n, d, ntb, out);
+    } else if (!wide) {
       auto kt = two ? k2 : k1;
       FUELG_CUDA(cudaFuncSetAttribute(kt, cudaFuncAttributeMaxDynamicSharedMemorySize, kTwoCtas));
       kt<<<dim3((unsigned)rb, (unsigned)((cb + strip - 1) / strip)), 256, two ? smem2 : smem1, stream>>>(
@@ -272,8 +380,8 @@ int pairwise_launch(const float* X, int64_t n, int d, int metric, int order, int
     }
     return ST_OK;
   };
-#define FUELG_PW(O, M, F)                                               \
-  FUELG_TRY(launch(pairwise_tile_kernel<O == ORDER_X86, M, F, 1>,       \
+#define FUELG_PW(O, M, F)                                                                        \
+  FUELG_TRY(launch(pairwise_rows_kernel<O, M, F>, pairwise_tile_kernel<O == ORDER_X86, M, F, 1>, \
                    pairwise_tile_kernel<O == ORDER_X86, M, F, 2>, pairwise_kernel<O, M, F>))
   const bool x86 = order == ORDER_X86, eu = metric == METRIC_EUCLIDEAN, cond = form == FUELG_PAIRWISE_CONDENSED;
   if (x86 && eu && cond) FUELG_PW(ORDER_X86, METRIC_EUCLIDEAN, FUELG_PAIRWISE_CONDENSED);
