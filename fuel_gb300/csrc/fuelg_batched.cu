@@ -445,6 +445,7 @@ __global__ void batched_step_kernel(int P, int32_t* __restrict__ pchg, int32_t* 
 }
 
 // Labels as the caller's 64-bit integers.
+constexpr int64_t kHostLabels = 16384;  // a problem, and that many more: fewer are widened on the host
 __global__ void widen_labels_kernel(const int32_t* __restrict__ labels, int64_t count, int64_t* __restrict__ out) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e < count) out[e] = labels[e];
@@ -2100,14 +2101,24 @@ extern "C" int fuelg_kmeans_batched(fuelg_kmeans_problem* probs, int32_t count, 
   std::vector<double> inert(P);
   FUELG_CUDA(cudaMemcpyAsync(conv.data(), dConv.p, sizeof(int32_t) * P, cudaMemcpyDeviceToHost, s));
   FUELG_CUDA(cudaMemcpyAsync(inert.data(), dInert.p, sizeof(double) * P, cudaMemcpyDeviceToHost, s));
-  // the labels are widened here and copied straight to the caller's arrays: as
+  // Many labels are widened here and copied straight to the caller's arrays: as
   // 32-bit integers through a host array, the copy, that array's fresh pages and one
-  // host loop took 18 ms of 71 for 20 million rows (6 now)
+  // host loop took 18 ms of 71 for 20 million rows (6 now).  Few come with the other
+  // results instead, in one copy, and the host widens them (as it does without room for
+  // the wide ones): a copy to an array costs 8 us, a label on the host 0.6 ns.  Calls, us,
+  // device / host: one problem of 3000 rows 303 / 291, 30 000 340 / 347, 65 000 332 / 365; 10
+  // of 10 000 554 / 530, of 30 000 629 / 719; 60 of 300 1012 / 516, of 5000 1658 / 1329, of
+  // 20 000 1945 / 2183.
   Scratch dLab64;
-  FUELG_TRY(dLab64.alloc(sizeof(int64_t) * ls, s));
-  widen_labels_kernel<<<(unsigned)((ls + 255) / 256), 256, 0, s>>>(dLab.as<int32_t>(), ls, dLab64.as<int64_t>());
-  note_launch();
-  FUELG_CUDA(cudaGetLastError());
+  std::vector<int32_t> lab32;
+  if (ls > kHostLabels * (P + 1) && dLab64.alloc(sizeof(int64_t) * ls, s) == ST_OK) {
+    widen_labels_kernel<<<(unsigned)((ls + 255) / 256), 256, 0, s>>>(dLab.as<int32_t>(), ls, dLab64.as<int64_t>());
+    note_launch();
+    FUELG_CUDA(cudaGetLastError());
+  } else {
+    lab32.resize(ls);
+    FUELG_CUDA(cudaMemcpyAsync(lab32.data(), dLab.p, sizeof(int32_t) * ls, cudaMemcpyDeviceToHost, s));
+  }
   // host centres leave by one copy (512 pageable ones take 4 ms)
   std::vector<float> hc((size_t)cs);
   FUELG_CUDA(cudaMemcpyAsync(hc.data(), dC.p, sizeof(float) * cs, cudaMemcpyDeviceToHost, s));
@@ -2141,21 +2152,26 @@ extern "C" int fuelg_kmeans_batched(fuelg_kmeans_problem* probs, int32_t count, 
       q.out_inertia = 0.0;
       continue;
     }
-    // The pages of an array that was never written are made here, by stores: the copy
-    // would have them made one by one on the device's side (54 ms for 160 MB; stores
-    // 5, and 5 the copy into present pages).
-    const size_t bytes = sizeof(int64_t) * (size_t)q.n;
-    volatile char* c = reinterpret_cast<volatile char*>(q.out_labels);
-    for (size_t e = 0; e < bytes; e += page) c[e] = 0;
-    c[bytes - 1] = 0;
-    FUELG_CUDA(cudaMemcpyAsync(q.out_labels, dLab64.as<int64_t>() + hp[p].lab_off, bytes, cudaMemcpyDefault, s));
-    d2h += (int64_t)bytes;
+    if (dLab64.p == nullptr) {
+      for (int64_t i = 0; i < q.n; i++) q.out_labels[i] = lab32[hp[p].lab_off + i];
+      d2h += (int64_t)sizeof(int32_t) * q.n;
+    } else {
+      // The pages of an array that was never written are made here, by stores: the
+      // copy would have them made one by one on the device's side (54 ms for 160 MB;
+      // stores 5, and 5 the copy into present pages).
+      const size_t bytes = sizeof(int64_t) * (size_t)q.n;
+      volatile char* c = reinterpret_cast<volatile char*>(q.out_labels);
+      for (size_t e = 0; e < bytes; e += page) c[e] = 0;
+      c[bytes - 1] = 0;
+      FUELG_CUDA(cudaMemcpyAsync(q.out_labels, dLab64.as<int64_t>() + hp[p].lab_off, bytes, cudaMemcpyDefault, s));
+      d2h += (int64_t)bytes;
+    }
     const int it = (!(flags & FUELG_LLOYD_FIXED_ITERS) && conv[p] > 0) ? conv[p] : max_iter;
     q.out_iters = it;
     q.out_inertia = inert[p];
     q.status = ST_OK;
   }
-  FUELG_CUDA(cudaStreamSynchronize(s));
+  if (dLab64.p != nullptr) FUELG_CUDA(cudaStreamSynchronize(s));
   if (stats) {
     float ms = 0.0f, hms = 0.0f;
     cudaEventElapsedTime(&ms, ev0, ev1);
