@@ -789,9 +789,22 @@ int exact_sums_step(ExactSums* s, const float* X, const int32_t* lab_new, int32_
 // 775 and 774; 100 000 x 10, k = 32 722 -> 582; 30 000 x 24, k = 64 681 for 701), up to
 // k d = 2560 means, which one block makes (5000 x 10, k = 250 624 -> 491; 1000 x 31, k = 256
 // 557 for 924).
+// Both read rows and centres from L1, a row or centre per lane, and give way earlier
+// where that is slow (small / tiled, us): rows that are multiples of 128 bytes, whose
+// lanes meet in the same banks (6288 x 32, k = 28 617 / 581, 12 014 x 32, k = 11 438 / 559;
+// 9046 x 64, k = 36 1470 / 679, 887 x 64, k = 93 739 / 812, 389 x 64, k = 192 1024 / 801), of
+// 64 bytes (9341 x 16, k = 107 811 / 660, 18 660 x 16, k = 33 523 / 585; 9413 x 48, k = 31 776 /
+// 611), of 16 and long (185 144 x 56, k = 2 1123 / 829, 28 284 x 56, k = 10 531 / 615), and
+// where the rows of a pass pass the L1s (206 673 x 38, k = 3 1461 / 1105, 157 645 x 50, k = 3
+// 1724 / 1208; 55 523 x 50, k = 5 541 / 690).
 bool exact_sums_assigns(int64_t n, int d, int k) {
-  return k <= kSmallMaxK && d <= kSmallMaxD &&
-         (double)n * k * d <= (k * d <= kOnePassSums ? kOnePassWork : kSmallWork);
+  if (k > kSmallMaxK || d > kSmallMaxD) return false;
+  const int64_t kd = (int64_t)k * d;
+  double limit = kd <= kOnePassSums ? kOnePassWork : kSmallWork;
+  if (d % 32 == 0) limit = kd <= 6144 ? 4e6 : 2e6;
+  else if (d % 16 == 0) limit = 1e7;
+  else if ((d % 4 == 0 && d >= 48) || (d >= 23 && (double)n * d > 3.6e6)) limit = std::min(limit, kSmallWork);
+  return (double)n * kd <= limit;
 }
 
 int exact_sums_assign_step(ExactSums* s, const float* X, const float* from, int order, int32_t* labels, bool first,
