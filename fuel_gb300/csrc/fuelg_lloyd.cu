@@ -45,7 +45,7 @@ struct ExactSums;
 ExactSums* exact_sums_new();
 void exact_sums_delete(ExactSums*);
 int exact_sums_init(ExactSums* s, const float* X, int64_t n, int d, int k, cudaStream_t stream);
-bool exact_sums_assigns(int64_t n, int d, int k);
+bool exact_sums_assigns(const ExactSums* s);
 int exact_sums_assign_step(ExactSums* s, const float* X, const float* from, int order, int32_t* labels, bool first,
                            bool write_centers, float* centers, int32_t* changed, cudaStream_t stream);
 int exact_sums_step(ExactSums* s, const float* X, const int32_t* lab_new, int32_t* labels, bool first,
@@ -428,7 +428,7 @@ int lloyd_run(const LloydParams& p, LloydResult* r, int* dev_status, cudaStream_
   if (exact) exact_sums_commit_view(es, &scv);
   auto pass = [&](bool first, bool write_centers, int32_t* chg) -> int {
     const bool fused = tc && exact && !first && d <= 1024;
-    const bool small = !tc && exact && exact_sums_assigns(n, d, k);
+    const bool small = !tc && exact && exact_sums_assigns(es);
     if (small) {
       if (p.tol > 0 && write_centers)
         FUELG_CUDA(cudaMemcpyAsync(cold.p, C, sizeof(float) * k * d, cudaMemcpyDeviceToDevice, stream));

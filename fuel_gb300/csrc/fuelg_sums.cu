@@ -131,6 +131,7 @@ constexpr int kSmallMaxK = 256, kSmallMaxD = 64;
 constexpr double kSmallWork = 1.6e7;    // n k d of assign_commit_kernel
 constexpr double kOnePassWork = 3.2e7;  // n k d of small_pass_kernel
 constexpr int64_t kOnePassSums = 2560;  // k d of small_pass_kernel
+constexpr double kDirectAdds = 2.5e6;   // n d L of small_pass_kernel without sums of its own
 constexpr int kAggCap = 2048;           // 64-bit sums of a block in shared memory (16 KB)
 template <int KIND, int ORDER>
 __global__ void __launch_bounds__(256) assign_commit_kernel(
@@ -780,6 +781,15 @@ int exact_sums_step(ExactSums* s, const float* X, const int32_t* lab_new, int32_
   return exact_sums_update(s, X, write_centers, centers, changed, cp, stream, false);
 }
 
+// Whether small_pass_kernel makes the sums: few means, and the first pass's adds (all
+// rows) in the blocks' own sums or few enough to meet at the global ones (5 passes of
+// 39 627 x 37, k = 21, 4.4 10^6 adds, 777 us, tiled 483; 20 000 x 37, k = 40, 2.2 10^6, 518 and 478,
+// 12 passes 803 and 811).
+static bool sums_in_one_pass(const ExactSums* s) {
+  const int64_t kd = (int64_t)s->k * s->d;
+  return kd <= kOnePassSums && (kd * s->L <= kAggCap || (double)s->n * s->d * s->L <= kDirectAdds);
+}
+
 // exact_sums_step with the assignment itself in the same kernel (assign_commit_kernel):
 // labels become the nearest of `from` by the exact arithmetic.
 // Up to n k d = 1.6 10^7 it is faster (12 passes: 2000 x 30, k = 32 653 -> 388 us; 5000 x 10,
@@ -794,16 +804,18 @@ int exact_sums_step(ExactSums* s, const float* X, const int32_t* lab_new, int32_
 // lanes meet in the same banks (6288 x 32, k = 28 617 / 581, 12 014 x 32, k = 11 438 / 559;
 // 9046 x 64, k = 36 1470 / 679, 887 x 64, k = 93 739 / 812, 389 x 64, k = 192 1024 / 801), of
 // 64 bytes (9341 x 16, k = 107 811 / 660, 18 660 x 16, k = 33 523 / 585; 9413 x 48, k = 31 776 /
-// 611), of 16 and long (185 144 x 56, k = 2 1123 / 829, 28 284 x 56, k = 10 531 / 615), and
-// where the rows of a pass pass the L1s (206 673 x 38, k = 3 1461 / 1105, 157 645 x 50, k = 3
-// 1724 / 1208; 55 523 x 50, k = 5 541 / 690).
-bool exact_sums_assigns(int64_t n, int d, int k) {
+// 611), of 16 (185 144 x 56, k = 2 1123 / 829, 28 284 x 56, k = 10 531 / 615; 60 passes of
+// 80 000 x 20, k = 20 2303 / 2089), and where the rows of a pass exceed the L1s (206 673 x 38,
+// k = 3 1461 / 1105, 157 645 x 50, k = 3 1724 / 1208; 55 523 x 50, k = 5 541 / 690).
+bool exact_sums_assigns(const ExactSums* s) {
+  const int64_t n = s->n;
+  const int d = s->d, k = s->k;
   if (k > kSmallMaxK || d > kSmallMaxD) return false;
   const int64_t kd = (int64_t)k * d;
-  double limit = kd <= kOnePassSums ? kOnePassWork : kSmallWork;
+  double limit = sums_in_one_pass(s) ? kOnePassWork : kSmallWork;
   if (d % 32 == 0) limit = kd <= 6144 ? 4e6 : 2e6;
   else if (d % 16 == 0) limit = 1e7;
-  else if ((d % 4 == 0 && d >= 48) || (d >= 23 && (double)n * d > 3.6e6)) limit = std::min(limit, kSmallWork);
+  else if ((d % 4 == 0 && d >= 16) || (d >= 23 && (double)n * d > 3.6e6)) limit = std::min(limit, kSmallWork);
   return (double)n * kd <= limit;
 }
 
@@ -817,7 +829,7 @@ int exact_sums_assign_step(ExactSums* s, const float* X, const float* from, int 
   int S = 1;
   while (S < 32 && S < k && 2 * S * n <= (int64_t)152 * 2048) S *= 2;
   const unsigned blocks = (unsigned)std::min<int64_t>((n * S + 255) / 256, 8 * 152);
-  if ((int64_t)k * s->d <= kOnePassSums) {
+  if (sums_in_one_pass(s)) {
     const int agg = (int64_t)k * s->d * s->L <= kAggCap ? 1 : 0;
     HotTimer* ht = hot_timer();
     if (ht) ht->begin(stream);
