@@ -29,7 +29,8 @@ namespace {
 
 constexpr int kThreads = 128;
 constexpr int kCB = 16;  // candidate buffer entries per thread, at most (kCbSmallK for small k)
-constexpr int64_t kTileMinRows = 1000;  // index rows from which exact_topk scans in register tiles
+constexpr int64_t kTileMinRows = 1000;   // index rows from which exact_topk scans in register tiles
+constexpr int64_t kTileMinRows1 = 4096;  // and for one key, which the scan below keeps in a register
 constexpr int kCbSmallK = 8;  // for kk <= 16: a smaller buffer leaves room for more resident CTAs
 
 struct ScanArgs {
@@ -372,8 +373,9 @@ int exact_topk(const ExactScanParams& p, uint64_t* out_keys, int* dev_status, cu
   // whose every key is merged: 100 000 queries, k = 5, d = 5 take 133 us here and
   // 326 in tiles at n = 100, 382 and 434 at n = 500; 200 000 queries, k = 20,
   // d = 2, n = 1000 take 1796 and 1163; 2000 queries, k = 10, d = 16, n = 2000
-  // take 170 and 111.
-  if (p.kind == KIND_KNN && p.n >= kTileMinRows && tile_scan_supported(p.d, p.kk)) {
+  // take 170 and 111.  One key costs the scan below no lists: 20 000 queries, d = 2, n =
+  // 2000 135 us here, 153 in tiles; 100 000, d = 2, n = 4200 790 and 486; 4000, d = 16 equal.
+  if (p.kind == KIND_KNN && p.n >= (p.kk == 1 ? kTileMinRows1 : kTileMinRows) && tile_scan_supported(p.d, p.kk)) {
     const int rc = tile_scan_topk(p, out_keys, dev_status, stream);
     if (rc != ST_ENOMEM) return rc;  // (without room for its lists: the scan below, whose are smaller)
   }

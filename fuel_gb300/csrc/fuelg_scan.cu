@@ -39,23 +39,30 @@ struct TileScanArgs {
   int tps;           // tiles staged per barrier
   uint64_t* out;     // [qblocks][J][8 W][kk]
   int J;
-  unsigned* gthr;    // [m] squared-distance limit bits shared by a query's runs, or nullptr
+  unsigned* gthr;    // [m] squared-distance limits (s_thr) shared by a query's runs, or nullptr
   f32x2 nz;          // kNegZero2 (tile_dists)
   int* status;
   const volatile int* cancel;
 };
 
 constexpr int kTileMaxD = 128;
+constexpr int kFewKeys = 8;  // keys of the kFew lists, at most
 // log entries that trigger a selection: a tile adds up to 128, warp_select takes 256
 constexpr int kTileLogCap = 32 * kSel - kTileP;
 constexpr int kTileSmemMax =
     (int)sizeof(float) * kTileMaxD * (kTileQS + 2 * kTilePS);  // 167 KB
 
-// SMALL: kk <= 32, each row's keys as a sorted list in shared memory that every
+// kSorted: kk <= 32, each row's keys as a sorted list in shared memory that every
 // passing key enters at once (the limit is never stale, so the fewest tiles
-// take the slow path); otherwise kept keys and an append log in global memory.
-template <bool FMA8, bool SMALL>
+// take the slow path); kFew: the same for kk <= kFewKeys, where a tile with many
+// candidates for a row hands in its smallest keys one by one until one does not enter,
+// in place of sorting them all (100 000 queries, k = 2, on 5000 x 2 rows ever closer to
+// them 4503 -> 1720 us, the per-thread lists 1499); kLogs: kept keys and an append log in
+// global memory.
+enum ScanLists { kLogs, kSorted, kFew };
+template <bool FMA8, ScanLists LISTS>
 __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileScanArgs a) {
+  constexpr bool SMALL = LISTS != kLogs, FEW = LISTS == kFew;
   extern __shared__ __align__(16) float tsm[];
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int QM = kTileQ * warps;
@@ -64,7 +71,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
   const size_t xtile = (size_t)a.d * kTilePS;
   const size_t xbuf = a.tps * xtile;
   constexpr int R = kTileQ * kTileMaxWarps;
-  // per query row: the bits of the largest squared distance that can still enter
+  // per query row: above the bits of every squared distance that can still enter
   __shared__ __align__(16) unsigned s_thr[R];
   __shared__ uint64_t s_list[SMALL ? R * 32 : 1];
   __shared__ uint64_t s_tau[SMALL ? 1 : R];                   // kk-th key held
@@ -76,13 +83,17 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
   int stop = 0;  // thread 0: the cancel word as of its last look
 
   // lane 0: row r's new limit from its kk-th key (never above what other runs of
-  // the query have found).  gthr has m words: rows past m, which keep index rows of
-  // zeros (see below), share no limit.
+  // the query have found); gthr has m words
   auto set_limit = [&](int r, int64_t q, uint64_t tau) {
     if (tau == KEY_NONE) return;
-    const unsigned lim = tile_limit_bits(key_dist(tau), a.metric);
-    s_thr[r] = min(s_thr[r], lim);
-    if (a.gthr != nullptr && q < a.m) atomicMin(a.gthr + q, lim);
+    const float D = key_dist(tau);
+    const unsigned lim = tile_limit_bits(D, a.metric);
+    const unsigned over = lim == 0xffffffffu ? lim : lim + 1;
+    // this run goes up in the index, so an equal distance no longer enters here; it can
+    // in another run (100 000 queries, k = 2, on 2000 x 2, each row some 50 times: 756 -> 298
+    // us with both, the per-thread lists 531)
+    s_thr[r] = min(s_thr[r], D == 0.0f ? 0u : a.metric == METRIC_SQEUCLIDEAN ? lim : over);
+    if (a.gthr != nullptr && q < a.m) atomicMin(a.gthr + q, over);
   };
   // folds row j's log into its kept keys (whole warp)
   auto flush = [&](int j, int64_t q0) {
@@ -112,8 +123,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
       tile_stage(xT + u * xtile, kTilePS, a.B, (x_first + u) * kTileP, kTileP, a.n, a.d, a.nb);
     if (lane < kTileQ) {
       const int r = warp * kTileQ + lane;
-      // (rows past m: their query is all zeros, so index rows of zeros are kept for
-      // them; nothing of theirs is written out)
+      // (rows past m: nothing enters)
       s_thr[r] = q0 + r >= a.m ? 0u : a.gthr != nullptr ? *((volatile unsigned*)a.gthr + q0 + r) : 0xffffffffu;
       if (!SMALL) {
         s_cnt[r] = s_len[r] = 0;
@@ -148,9 +158,9 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
         const uint4 th0 = *reinterpret_cast<const uint4*>(s_thr + warp * kTileQ);
         const uint4 th1 = *reinterpret_cast<const uint4*>(s_thr + warp * kTileQ + 4);
         const unsigned thr[kTileQ] = {th0.x, th0.y, th0.z, th0.w, th1.x, th1.y, th1.z, th1.w};
-        unsigned hits = 0;  // rows with a distance at or below their limit
+        unsigned hits = 0;  // rows with a distance below their limit
 #pragma unroll
-        for (int j = 0; j < kTileQ; j++) hits |= tile_min_bits(s[j]) <= thr[j] ? 1u << j : 0u;
+        for (int j = 0; j < kTileQ; j++) hits |= tile_min_bits(s[j]) < thr[j] ? 1u << j : 0u;
         hits = __reduce_or_sync(0xffffffffu, hits);
         while (hits) {
           const int j = __ffs(hits) - 1;
@@ -182,16 +192,47 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
           int found = 0;
 #pragma unroll
           for (int i = 0; i < 4; i++) {
-            in[i] = __ballot_sync(0xffffffffu, __float_as_uint(v[i]) <= lim && 32 * i < left);
+            in[i] = __ballot_sync(0xffffffffu, __float_as_uint(v[i]) < lim && 32 * i < left);
             found += __popc(in[i]);
           }
           if (SMALL) {
             uint64_t kept = s_list[r * 32 + lane];
             uint64_t tau = shfl_u64(kept, a.kk - 1);
+            if (FEW && found > 12) {
+              // many candidates for few places (an index's first tiles, rows ever closer to
+              // the query): the smallest keys one after the other, until one does not enter
+              unsigned u[4];
+#pragma unroll
+              for (int i = 0; i < 4; i++) {
+                const float dv = a.metric == METRIC_EUCLIDEAN ? __fsqrt_rn(v[i]) : v[i];
+                u[i] = in[i] >> lane & 1 ? __float_as_uint(dv) : 0xffffffffu;
+              }
+              for (;;) {
+                const unsigned w = __reduce_min_sync(0xffffffffu, min(min(u[0], u[1]), min(u[2], u[3])));
+                if (w == 0xffffffffu || w > (uint32_t)(tau >> 32)) break;
+                int at = 0;  // the lowest column that holds it
+#pragma unroll
+                for (int i = 3; i >= 0; i--) {
+                  const unsigned b = __ballot_sync(0xffffffffu, u[i] == w);
+                  if (b) at = __ffs(b) - 1 + 32 * i;
+                }
+                const uint64_t key = ((uint64_t)w << 32) | (uint32_t)(p0 + at);
+                if (key >= tau) break;
+                kept = warp_insert32(kept, key, lane);
+                tau = shfl_u64(kept, a.kk - 1);
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                  if (at == lane + 32 * i) u[i] = 0xffffffffu;
+              }
+              s_list[r * 32 + lane] = kept;
+              if (lane == 0) set_limit(r, q0 + r, tau);
+              __syncwarp();
+              continue;
+            }
 #pragma unroll
             for (int i = 0; i < 4; i++) {
               if (in[i] == 0) continue;
-              if (found > 12) {
+              if (!FEW && found > 12) {
                 const float dv = a.metric == METRIC_EUCLIDEAN ? __fsqrt_rn(v[i]) : v[i];
                 kept = warp_merge32(kept, in[i] >> lane & 1 ? make_key(dv, (uint32_t)(p0 + lane + 32 * i)) : KEY_NONE,
                                     lane);
@@ -308,8 +349,10 @@ bool tile_scan_supported(int d, int kk) { return d >= 1 && d <= kTileMaxD && kk 
 int tile_scan_topk(const ExactScanParams& p, uint64_t* out_keys, int* dev_status, cudaStream_t stream) {
   const bool fma = p.order == ORDER_X86;
   const bool small = p.kk <= 32;
-  auto kern = small ? (fma ? scan_tile_kernel<true, true> : scan_tile_kernel<false, true>)
-                    : (fma ? scan_tile_kernel<true, false> : scan_tile_kernel<false, false>);
+  const bool few = p.kk <= kFewKeys;
+  auto kern = few ? (fma ? scan_tile_kernel<true, kFew> : scan_tile_kernel<false, kFew>)
+              : small ? (fma ? scan_tile_kernel<true, kSorted> : scan_tile_kernel<false, kSorted>)
+                      : (fma ? scan_tile_kernel<true, kLogs> : scan_tile_kernel<false, kLogs>);
   const int64_t nt = (p.n + kTileP - 1) / kTileP;
   const int lstride = p.kk + kTileLogCap + kTileP;
   // tiles per barrier: several of short rows, so that a warp with more candidates
