@@ -1195,7 +1195,8 @@ int fuelg_knn_f64(fuelg_index* ix, const double* queries, int64_t m, int32_t k, 
   OutBuf oi, od;
   FUELG_TRY(oi.init(out_idx, (size_t)m * k * sizeof(int64_t), s));
   FUELG_TRY(od.init(out_dist, (size_t)m * k * sizeof(double), s));
-  if (!ix->screen_tried && f64_screen_serves(ix->n, ix->d, m)) {
+  const int64_t kk = std::min<int64_t>(exclude_mode == FUELG_EXCLUDE_NONE ? k : (int64_t)k + 1, ix->n);
+  if (!ix->screen_tried && f64_screen_serves(ix->n, ix->d, m, kk)) {
     FUELG_TRY(f64_screen_build(ix->X64, ix->n, ix->d, s, &ix->screen));
     ix->screen_tried = true;
   }

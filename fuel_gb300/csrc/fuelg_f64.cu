@@ -615,14 +615,23 @@ void f64_screen_free(F64Screen* f) {
   delete f;
 }
 
-// The screen's launches cost about 40 us more than the FP64 scan's, which a few
-// pairs do not repay.  Measured (us a call, FP64 scan / screen, k = 10): one
-// query, d = 16: n = 5000 59 / 82, 10 000 75 / 85, 20 000 104 / 84, 10^5 525 / 94;
-// m = 100, n = 2000, d = 16: 78 / 108, m = 300: 126 / 111; m = n = 1000, d = 2:
-// 102 / 104, d = 8: 135 / 106; m = n = 20 000, d = 16: 53 800 / 1210.
-bool f64_screen_serves(int64_t n, int d, int64_t m) {
-  return n >= 1000 && n < (1ll << 31) && tile_scan_supported(d, 1) &&
-         (n >= 16384 || (double)m * n * d >= 8e6);
+// Candidates kept for kk keys: ranks beyond them for the proof's error bound to fall
+// between (kk <= 28 then still fits the tile scan's sorted lists of 32).
+static int64_t screen_keys(int64_t kk) { return kk + std::max<int64_t>(4, kk / 8); }
+
+// Whether the screen is the faster: what the FP64 scan takes longer, in us (its distances
+// at the FP64 rate, one block's passes over a query's distances, and all queries'),
+// against the screen's launches, and its logs and ranking above 32 candidates, which few
+// queries make little of.  Fitted to 900 calls timed both ways (random rows, n 1000 to
+// 40 000, k 5 to 200): the slower way is taken by more than 4 % in 6 of them where that
+// is the screen, by 13 % at most, and in 22 where it is the scan.  (Scan / screen: 157 x
+// 1158 x 59, k = 200 134 / 357 us; 300 x 2000 x 16, k = 10 126 / 111; 1 x 20 000 x 16 104 / 84;
+// 20 000 x 20 000 x 16 53 800 / 1210.)
+bool f64_screen_serves(int64_t n, int d, int64_t m, int64_t kk) {
+  if (n < 1000 || n >= (1ll << 31) || !tile_scan_supported(d, 1)) return false;
+  const double rows = n * 1e-3, pairs = (double)m * n * 1e-6;
+  if (screen_keys(kk) <= 32) return 5.6 * pairs * d + 3.8 * rows + 31.0 * pairs >= 48.0 + 0.3 * d;
+  return 4.6 * pairs * d + 3.8 * rows + 25.0 * pairs >= 80.0 + (double)kk + 0.4 * d - (m <= 4 ? 30.0 : 0.0);
 }
 
 int f64_screen_build(const double* X, int64_t n, int d, cudaStream_t s, F64Screen** out) {
@@ -703,10 +712,8 @@ int f64_knn(const F64Scan& x, const double* Q, int64_t m, int k, int mode, int64
     FUELG_CUDA(cudaGetLastError());
     return ST_OK;
   }
-  // candidates kept beyond kk: ranks for the proof's error bound to fall between
-  // (kk <= 28 then still fits the tile scan's sorted lists of 32)
-  const int64_t kk2 = kk + std::max<int64_t>(4, kk / 8);
-  if (x.screen == nullptr || !f64_screen_serves(x.n, x.d, m) ||
+  const int64_t kk2 = screen_keys(kk);
+  if (x.screen == nullptr || !f64_screen_serves(x.n, x.d, m, kk) ||
       !tile_scan_supported(x.d, (int)std::min<int64_t>(kk2, 1 << 20)) || m >= (1ll << 31))
     return f64_knn_scan(x, Q, m, nullptr, kk, k, mode, out_idx, out_dist, s);
   // query batches: their copies, candidates and redo lists stay below ~1 GiB

@@ -243,7 +243,7 @@ int exact_knn_in_scratch(const ExactScanParams& p, int k, int exclude_mode, int6
 struct F64Screen;
 // Rounded copy of a float64 index for the FP32 screen of its kNN calls; *out
 // stays nullptr where its values do not allow one.  Shapes: f64_screen_serves.
-bool f64_screen_serves(int64_t n, int d, int64_t m);
+bool f64_screen_serves(int64_t n, int d, int64_t m, int64_t kk);
 int f64_screen_build(const double* X, int64_t n, int d, cudaStream_t s, F64Screen** out);
 void f64_screen_free(F64Screen* f);
 struct F64Scan {
