@@ -553,7 +553,7 @@ def knn_plain_rate(lib, _lib, torch, args, parity=False):
                "precision": "fp32",
                "e2e": {"queries_per_s": n / (te / 1e3), "ms_per_call": te, "h2d_bytes_per_call": n * d * 4,
                        "d2h_bytes_per_call": n * k * 12},
-               "roofline": plain_roofline(lib, _lib, n * n, d, hk, "scan_topk_kernel (exact FP32 kNN scan)")}
+               "roofline": plain_roofline(lib, _lib, n * n, d, hk, "scan_tile_kernel (exact FP32 kNN scan)")}
         out["fp64"] = error_report(lib, _lib, h, _lib.ptr(Qd), n, k, _lib.ptr(oi), _lib.ptr(od))
         if parity:
             from oracle import oracle
@@ -667,7 +667,7 @@ def knn_tc_rate(lib, _lib, torch, args, m_tc=None, plain=True, reps=1, n_index=K
             p_hot = st.hot_kernel_ms
             out["plain_fp32"] = {"queries": mp, "ms_per_call": st.device_ms, "distance_evals_per_s": pr,
                                  "roofline": plain_roofline(lib, _lib, mp * n, d, p_hot,
-                                                            "scan_topk_kernel (exact FP32 kNN scan)")}
+                                                            "scan_tile_kernel (exact FP32 kNN scan)")}
             out["tc_vs_plain"] = out["distance_evals_per_s"] / pr
         return out
     finally:

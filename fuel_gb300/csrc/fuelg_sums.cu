@@ -427,7 +427,6 @@ __device__ __forceinline__ float mean_elem(unsigned long long* __restrict__ limb
   return mean_of<L>(lp, lv, counts[(int)(e / d)], e_lo, centers + e, centers[e], write_centers);
 }
 
-// Hand the change count to the host and reset the per-pass counters.
 // Few sums: a whole pass in one launch.  As assign_commit_kernel, but a changed
 // point's coordinates go straight to the sums -- its S lanes share them, one atomic
 // per 32-bit slice, into the block's own sums where they fit (agg) and those into the
@@ -528,6 +527,7 @@ __global__ void __launch_bounds__(256) small_pass_kernel(
   }
 }
 
+// Hand the change count to the host and reset the per-pass counters.
 __device__ __forceinline__ void mean_handoff(int bid, int nblk, int32_t* __restrict__ nchg,
                                              int32_t* __restrict__ changed, int32_t* __restrict__ zero4k, int nzero) {
   if (bid == 0 && threadIdx.x == 0) {

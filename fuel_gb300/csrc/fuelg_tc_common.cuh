@@ -43,24 +43,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Two IEEE fused multiply-adds in one paired instruction: (a0, a1) <-
-// (fma(a0, b, c0), fma(a1, b, c1)).  Each half is exactly the scalar fmaf.
-__device__ __forceinline__ void fma2_rn(uint32_t& a0, uint32_t& a1, float b, float c0, float c1) {
-  unsigned long long x, y, z;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "r"(a0), "r"(a1));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b), "f"(b));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(z) : "f"(c0), "f"(c1));
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(z) : "l"(x), "l"(y));
-  asm("mov.b64 {%0, %1}, %2;" : "=r"(a0), "=r"(a1) : "l"(z));
-}
-// Smallest of three floats in one instruction (a NaN operand is ignored, as
-// fminf ignores it).
-__device__ __forceinline__ float min3_f32(float a, float b, float c) {
-  float r;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-
 // Largest of three floats in one instruction (a NaN operand is ignored).
 __device__ __forceinline__ float max3_f32(float a, float b, float c) {
   float r;
@@ -94,13 +76,6 @@ inline uint64_t pipeline_wait_ns() {
     if (v >= 1) return (uint64_t)v < kWaitNs ? (uint64_t)v : kWaitNs;
   }
   return kWaitNs;
-}
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, int x, int y, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
 }
 // Contiguous bytes global -> shared (one bulk copy; dst, src 16-byte aligned,
 // bytes a multiple of 16), completing `bytes` of transaction on bar.
@@ -198,16 +173,6 @@ __device__ __forceinline__ void named_bar_sync(int bar_id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(bar_id), "r"(nthreads) : "memory");
 }
 
-__device__ __forceinline__ int named_bar_or(int bar_id, int nthreads, int v) {
-  int r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.or.pred q, %2, %3, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"(v), "r"(bar_id), "r"(nthreads)
-      : "memory");
-  return r;
-}
-
 // tcgen05.ld of 16 columns without the completion wait (pair with tmem_ld_wait)
 __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -256,20 +221,6 @@ __device__ __forceinline__ void tmem_regs_ready(uint32_t (&r)[16]) {
                  "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
                  "+r"(r[15]));
 }
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
-}
-
 
 int make_map_bf16(CUtensorMap* tm, const void* ptr, int64_t rows, int row_elems, int box_rows);
 // Rows of 16 two-byte elements, 32-byte swizzle.
