@@ -83,7 +83,8 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
   int stop = 0;  // thread 0: the cancel word as of its last look
 
   // lane 0: row r's new limit from its kk-th key (never above what other runs of
-  // the query have found); gthr has m words
+  // the query have found).  gthr has m words, and q < m: rows past m have the limit 0,
+  // which no distance is below, so they never hold a key (see the start of a piece).
   auto set_limit = [&](int r, int64_t q, uint64_t tau) {
     if (tau == KEY_NONE) return;
     const float D = key_dist(tau);
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
     // in another run (100 000 queries, k = 2, on 2000 x 2, each row some 50 times: 756 -> 298
     // us with both, the per-thread lists 531)
     s_thr[r] = min(s_thr[r], D == 0.0f ? 0u : a.metric == METRIC_SQEUCLIDEAN ? lim : over);
-    if (a.gthr != nullptr && q < a.m) atomicMin(a.gthr + q, over);
+    if (a.gthr != nullptr) atomicMin(a.gthr + q, over);
   };
   // folds row j's log into its kept keys (whole warp)
   auto flush = [&](int j, int64_t q0) {
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(32 * kTileMaxWarps, 2) scan_tile_kernel(TileSc
       tile_stage(xT + u * xtile, kTilePS, a.B, (x_first + u) * kTileP, kTileP, a.n, a.d, a.nb);
     if (lane < kTileQ) {
       const int r = warp * kTileQ + lane;
-      // (rows past m: nothing enters)
+      // (rows past m: nothing is below 0, so nothing enters)
       s_thr[r] = q0 + r >= a.m ? 0u : a.gthr != nullptr ? *((volatile unsigned*)a.gthr + q0 + r) : 0xffffffffu;
       if (!SMALL) {
         s_cnt[r] = s_len[r] = 0;
