@@ -613,6 +613,14 @@ void tune_store_locked(const TuneKey& key, int tier) {
   }
 }
 
+// Index rows below which the plain scan is a candidate too: few tiles, most of whose
+// columns the tensor-core screen logs.  Which is faster depends on the number of queries
+// there (k = 150 on 1400 x 40: 300 queries 1011 us, the plain scan 178, 10 000 1226 and 690;
+// k = 20 on 3000 x 200: 507 and 275, 567 and 2343), so their buckets have it too, in steps of
+// four, and up to kPlainAutoQueries rows are timed; above them the tensor-core tiers
+// alone are.
+constexpr int64_t kPlainAutoRows = 4096, kPlainAutoQueries = 32768;
+
 // The tier a FUELG_PREC_AUTO kNN call runs.  Called with ix->mu held.
 int resolve_knn_precision(fuelg_index* ix, const float* Q, int64_t m, int kk, int* dstat, cudaStream_t s,
                           int* out) {
@@ -625,7 +633,9 @@ int resolve_knn_precision(fuelg_index* ix, const float* Q, int64_t m, int kk, in
     *out = FUELG_PREC_BF16;  // exact operands: one product, no re-score where the screen is exact
     return ST_OK;
   }
-  const TuneKey key{ix->d, ilog2_floor(ix->n), ilog2_floor(2 * (int64_t)kk - 1), cls};
+  const bool plain = ix->n < kPlainAutoRows && m <= kPlainAutoQueries;
+  const TuneKey key{ix->d, ilog2_floor(ix->n), ilog2_floor(2 * (int64_t)kk - 1),
+                    plain ? cls + 16 * (1 + ilog2_floor(m) / 2) : cls};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     tune_load_locked();
@@ -637,29 +647,30 @@ int resolve_knn_precision(fuelg_index* ix, const float* Q, int64_t m, int kk, in
   }
   // time the eligible tiers on the first rows of this call (each run twice:
   // the first builds the tier's index copy and warms up)
-  const int64_t mt = std::min<int64_t>(m, 4096);
+  const int64_t mt = std::min<int64_t>(m, plain ? kPlainAutoQueries : 4096);
   Scratch keys;
   FUELG_TRY(keys.alloc((size_t)mt * kk * sizeof(uint64_t), s));
-  const int cand_f16[3] = {FUELG_PREC_F16, FUELG_PREC_SPLIT_BF16, FUELG_PREC_BF16};
-  const int cand_wide[2] = {FUELG_PREC_SPLIT_BF16, FUELG_PREC_BF16};
-  const int* cand = cls == TC_CLASS_F16_RANGE ? cand_f16 : cand_wide;
-  const int nc = cls == TC_CLASS_F16_RANGE ? 3 : 2;
-  int best = FUELG_PREC_FP32;
+  std::vector<int> cand;
+  if (cls == TC_CLASS_F16_RANGE) cand.push_back(FUELG_PREC_F16);
+  cand.push_back(FUELG_PREC_SPLIT_BF16);
+  cand.push_back(FUELG_PREC_BF16);
+  if (plain) cand.push_back(FUELG_PREC_FP32);
+  int best = -1;
   float best_ms = 1e30f;
-  for (int c = 0; c < nc; c++) {
+  for (const int c : cand) {
     int used = 0;
     int64_t resc = 0;
-    FUELG_TRY(index_topk(ix, Q, mt, kk, cand[c], keys.as<uint64_t>(), dstat, s, &used, &resc));
+    FUELG_TRY(index_topk(ix, Q, mt, kk, c, keys.as<uint64_t>(), dstat, s, &used, &resc));
     Timer tm(s);
-    FUELG_TRY(index_topk(ix, Q, mt, kk, cand[c], keys.as<uint64_t>(), dstat, s, &used, &resc));
+    FUELG_TRY(index_topk(ix, Q, mt, kk, c, keys.as<uint64_t>(), dstat, s, &used, &resc));
     const float ms = (float)tm.stop();
-    if (used == cand[c] && ms < best_ms) {
+    if (used == c && ms < best_ms) {
       best_ms = ms;
-      best = cand[c];
+      best = c;
     }
   }
+  if (best < 0) return ST_OK;  // none ran (this call's values or memory): not the bucket's answer
   *out = best;
-  if (best == FUELG_PREC_FP32) return ST_OK;  // none ran (this call's values or memory): not the bucket's answer
   std::lock_guard<std::mutex> lk(g_tune_mu);
   tune_store_locked(key, best);
   return ST_OK;

@@ -66,8 +66,9 @@ extern "C" {
    range / serving: d outside [32, 256] -> FP32; integer data with |v| <= 256
    -> BF16 (it holds them exactly); otherwise the fastest of the eligible
    tensor-core tiers, timed on the call's first (up to) 4096 query rows the
-   first time a (d, log2 n, log2 k, value class) bucket is seen, and kept for
-   the process -- and in the file named by FUELG_TUNE_CACHE when that variable
+   first time a (d, log2 n, log2 k, value class) bucket is seen; for fewer than
+   4096 index rows and up to 32768 queries FP32 is timed too, on all rows, and
+   the bucket has log4 m.  The choice is kept for the process -- and in the file named by FUELG_TUNE_CACHE when that variable
    is set, one line per bucket.  k-means: the split-BF16 tier where its screen
    serves the shape (d >= 32) and the problem is large enough (n >= 16384),
    else FP32; batched k-means: split-BF16 for the problems it serves.
