@@ -61,6 +61,10 @@ constexpr int kNB = 16;         // columns of the norm operand: one K step
 constexpr uint32_t kNormBytes = XN * kNB * 2;  // its 4 KB tile
 constexpr int kMaxStages = 12;  // index tiles in shared memory, at most
 constexpr int kMinQuantum = 16;  // tiles of a piece, at least
+// Index tiles below which a piece may have two: 300 queries, FP16, k = 20 / 150, on 1400 x 100
+// 360 / 1129 us in one piece a block, 319 / 892 in four, 333 / 552 in eleven; on 3000 x 100 476 /
+// 1100 and, twelve pieces, 327 / 612; 10 000 queries, k = 150, on 3000 x 200 1747 and, three, 1451.
+constexpr int kSmallIndex = 64;
 // Each query row has two logs of screened (value, column) pairs: its epilogue lane
 // fills one while a selection warp folds the other into the row's kept keys.
 constexpr int kLog = 192;      // pairs per log: a step adds up to 32
@@ -1498,7 +1502,7 @@ int knn_tc_topk(const TcIndex* ti, const float* Q32, int64_t m, const float* X32
   // query count, or the last part of a large one) would leave slots idle, so
   // there each block's index scan is cut into s equal tile ranges (quanta);
   // the quanta, block-major, are dealt out L at a time to consecutive CTAs,
-  // L = ceil(quanta / slots).  s is the count (quanta of >= kMinQuantum tiles, at most
+  // L = ceil(quanta / slots).  s is the count (quanta of >= kMinQuantum tiles, or 2, at most
   // kMaxSplits - 2 pieces per block) that minimises the longest CTA's work,
   // L (ntiles / s + 4) tiles with 4 tiles' worth charged per piece for its
   // pipeline refill and its list's start, and 15% more for pieces that a CTA works
@@ -1513,7 +1517,10 @@ int knn_tc_topk(const TcIndex* ti, const float* Q32, int64_t m, const float* X32
     int best = 1;
     double best_cost = 0.0;
     for (int sq = 1; sq <= kMaxQuanta; sq++) {
-      if (sq > 1 && ntiles_all / sq < kMinQuantum) break;
+      // (a small index is all first tiles, whose columns are logged: what bounds it is
+      // each CTA's selection, so it is spread as far as every piece has a CTA of its own)
+      const bool spread_out = ntiles_all < kSmallIndex && qbl * sq <= slots;
+      if (sq > 1 && ntiles_all / sq < (spread_out ? 2 : kMinQuantum)) break;
       const int64_t L = (qbl * sq + slots - 1) / slots;
       const double cost = (double)L * ((double)ntiles_all / sq + 4.0) * (L > 1 ? 1.15 : 1.0);
       if (sq == 1 || cost < best_cost) best = sq, best_cost = cost;
