@@ -215,8 +215,9 @@ __device__ __forceinline__ f32x2 exact_dist_pair(const f32x2 (&x)[D], const f32x
 // registers; others take fuel's order from memory) whose centres fit the stage, up to
 // 8192 and 2048: two centres per packed step, their coordinates interleaved in shared
 // memory; with more centres one at a time, from global memory (10 passes of 100 000 x 2,
-// k = 8200 9.1 ms, 200 000 x 8, k = 2100 9.7; 29.5 and 35.7 through the general loop).  WIDE: some problem has 32 or 64 dimensions, whose rows are held in
-// registers (128 per thread; 64 without).  Bound by FP32 issue and, in the first
+// k = 8200 9.1 ms, 200 000 x 8, k = 2100 9.7; 29.5 and 35.7 through the general loop).
+// WIDE: some problem has 32 dimensions or more (rows of 32 and 64 are held in
+// registers): 128 registers per thread; 64 without.  Bound by FP32 issue and, in the first
 // passes, by the adds of changed rows: a later pass over 10.3 million rows of 2 or
 // 8 dimensions, k to 256: 0.90 -> 0.56 ms against one centre at a time.
 template <int KIND, int ORDER, bool WIDE>

@@ -6,8 +6,8 @@
 // they come; the keys are unique, so the sort by (distance, index) that the result
 // needs anyway makes the order definite.  The counts' prefix sums are the result's
 // offsets, and one warp (above 256 hits: one block) sorts a query's slots into its
-// place.  Only when a query has more hits than slots does a second pass fill the
-// lists at their offsets, for a segmented sort.
+// place.  Only when a query has more hits than slots, or there is no room for slots,
+// does a second pass fill the lists at their offsets, for a segmented sort.
 #include <algorithm>
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_segmented_sort.cuh>
@@ -25,8 +25,8 @@ constexpr int kRangeMaxD = 128;
 constexpr int kMaxStrip = 8;                // most 128-row tiles that one CTA works through
 constexpr int kTwoPerSm = 2 * 152;          // places on the chip with two CTAs per SM
 constexpr int kTwoCtas = 112 * 1024;        // shared memory with which two CTAs fit an SM
-// Most slots of a query: what a block sorts in the shared memory that lets six
-// blocks share an SM.  (With 1024 the 300-hit self-join had rows past them and took
+// Most slots of a query: what range_long_kernel's block sorts in 34 KB of shared
+// memory.  (With 1024 the 300-hit self-join had rows past them and took
 // 4.29 ms for 1.74.)
 constexpr int kSlots = 4096;
 constexpr int kWarpSort = 256;              // most keys that a warp sorts

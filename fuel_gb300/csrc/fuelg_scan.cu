@@ -7,7 +7,7 @@
 // registers, a row's 128 distances of a tile are tested against its running
 // kk-th key with one vote, the few that pass are appended to the row's log, and
 // the log is folded into the row's kept keys by the warp (a sorted list of
-// 32 keys merged bitonically for kk <= 32, warp_select above).  The lists of a
+// 32 keys merged bitonically for kk <= 32, few keys one by one, warp_select above).  The lists of a
 // query block's runs are merged afterwards.
 //
 // Bound: FP32 issue (3 operations per pair and dimension, one fold per 8): 47

@@ -7,7 +7,7 @@ libfuelg.so; distances are bit-identical to fuel's f32 distances for the
 chosen summation profile (``order``).
 
 What is served: float32 data and float64 data (every other input dtype
-becomes float64, as in fuel; float64 runs the exact FP64 scan with fuel's f64
+becomes float64, as in fuel; float64 gives fuel's exact f64
 distances), distances ``euclidean``/``l2`` and ``sqeuclidean``/
 ``squared_euclidean``, the linear scan (``tree`` = ``None``, ``'auto'``,
 ``'linear'``, ``'brute'``, ``'bruteforce'``).  Anything else raises

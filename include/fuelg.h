@@ -68,14 +68,14 @@ extern "C" {
    tensor-core tiers, timed on the call's first (up to) 4096 query rows the
    first time a (d, log2 n, log2 k, value class) bucket is seen; for fewer than
    4096 index rows and up to 32768 queries FP32 is timed too, on all rows, and
-   the bucket has log4 m.  The choice is kept for the process -- and in the file named by FUELG_TUNE_CACHE when that variable
-   is set, one line per bucket.  k-means: the split-BF16 tier where its screen
+   the bucket has log4 m.  The choice is kept for the process -- and in the file named
+   by FUELG_TUNE_CACHE when that variable is set, one line per bucket.  k-means: the split-BF16 tier where its screen
    serves the shape (d >= 32) and the problem is large enough (n >= 16384),
    else FP32; batched k-means: split-BF16 for the problems it serves.
    fuelg_stats.precision_used reports what ran. */
 #define FUELG_PREC_AUTO (-1)
-/* Reported in fuelg_stats.precision_used by the float64 calls (the exact FP64
-   scan); not a request value. */
+/* Reported in fuelg_stats.precision_used by the float64 calls (exact FP64
+   distances); not a request value. */
 #define FUELG_PREC_FP64 5
 
 #define FUELG_LLOYD_FIXED_ITERS 1 /* run exactly max_iter iterations (ignore changed==0 stop) */
@@ -223,9 +223,12 @@ int fuelg_pairwise(const float *X, int64_t n, int32_t d, int32_t metric, int32_t
  * (python/fuel/_dispatch.py:8-19; build_linear_scan_f64, python/search.rs:
  * 1371-1389) and compares f64 distances in its f64 operation order
  * (src/distance/squared_euclidean.rs:44-67 on x86 AVX + FMA builds, :99-133
- * elsewhere; Euclidean = f64 sqrt).  These calls run the exact FP64 scan:
- * every (query, point) distance in that order, (distance, index) order and
- * the same tie, exclude and padding rules as the float32 calls.  A float64
+ * elsewhere; Euclidean = f64 sqrt).  Results are those of the FP64 scan: every
+ * (query, point) distance in that order, (distance, index) order and the same
+ * tie, exclude and padding rules as the float32 calls.  The first kNN call large
+ * enough for it adds a float32 copy of the rows (4 n d bytes) to the index, with
+ * which a screen leaves few pairs to FP64; a query whose answer the screen cannot
+ * prove, and every call where there is no room, takes the scan itself.  A float64
  * index (n <= 2^32 - 2) serves only the _f64 calls, a float32 index only the
  * float32 calls (FUELG_EINVAL otherwise).  Distances are f64 (+inf padding);
  * fuelg_stats.precision_used reports FUELG_PREC_FP64. */
